@@ -14,14 +14,33 @@ DEFAULT_LIB_PATH = os.path.join(_PKG, "libamsim.so")
 # build libamsim_check.so (build_checked below); it is never rebuilt automatically.
 LIB_PATH = os.environ.get("AMSIM_LIBRARY") or DEFAULT_LIB_PATH
 CHECKED_LIB_PATH = os.path.join(_PKG, "libamsim_check.so")
-SOURCES = [os.path.join(_PKG, "csrc", "amsim.cu")]
-HEADERS = [os.path.join(_PKG, "csrc", "amsim_kernels.cuh"), os.path.join(_PKG, "csrc", "amsim_wide.cuh"),
+SOURCES = [os.path.join(_PKG, "csrc", "amsim.cu"), os.path.join(_PKG, "csrc", "amsim_codes.cu")]
+HEADERS = [os.path.join(_PKG, "csrc", h) for h in ("amsim_kernels.cuh", "amsim_wide.cuh", "amsim_codes.cuh", "amsim_codes_launch.h",
+                                                   "amsim_factor.h")] + [
            os.path.join(os.path.dirname(_PKG), "include", "amsim.h")]
 
 NVCC_FLAGS = [
-    "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-shared", "-Xcompiler", "-fPIC",
+    "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-DAMSIM_SPLIT_TU",
 ]
+
+
+def _compile(out: str, extra=(), only_stale=False) -> None:
+    """The sources side by side (one nvcc each), then one link."""
+    nvcc = os.environ.get("NVCC", "nvcc")
+    tmp = os.path.join(_PKG, "build", os.path.basename(out))
+    os.makedirs(tmp, exist_ok=True)
+    objs, jobs = [], []
+    for src in SOURCES:
+        obj = os.path.join(tmp, os.path.basename(src) + ".o")
+        objs.append(obj)
+        deps = [src] + HEADERS
+        if only_stale and os.path.exists(obj) and all(os.path.getmtime(d) <= os.path.getmtime(obj) for d in deps):
+            continue
+        jobs.append((src, subprocess.Popen([nvcc] + NVCC_FLAGS + list(extra) + ["-c", "-o", obj, src])))
+    failed = [src for src, job in jobs if job.wait() != 0]
+    if failed:
+        raise RuntimeError(f"nvcc failed on {failed}")
+    subprocess.check_call([nvcc] + NVCC_FLAGS + ["-shared", "-o", out] + objs)
 
 
 def needs_build() -> bool:
@@ -56,17 +75,14 @@ def build_checked(force: bool = False) -> str:
     AMSIM_LIBRARY=<path>; read the verdict with amsim_debug_bounds_report()."""
     if force or not os.path.exists(CHECKED_LIB_PATH) or any(
             os.path.getmtime(f) > os.path.getmtime(CHECKED_LIB_PATH) for f in SOURCES + HEADERS if os.path.exists(f)):
-        nvcc = os.environ.get("NVCC", "nvcc")
-        subprocess.check_call([nvcc] + NVCC_FLAGS + ["-DAMSIM_BOUNDS_CHECK", "-o", CHECKED_LIB_PATH] + SOURCES)
+        _compile(CHECKED_LIB_PATH, ["-DAMSIM_BOUNDS_CHECK"])
     return CHECKED_LIB_PATH
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     """Build libamsim.so (and the C driver) if missing or older than the sources."""
     if force or needs_build():
-        nvcc = os.environ.get("NVCC", "nvcc")
-        cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", DEFAULT_LIB_PATH] + SOURCES
-        subprocess.check_call(cmd)
+        _compile(DEFAULT_LIB_PATH, ["-Xptxas", "-v"] if verbose else [])
     if force or not os.path.exists(DRIVER_PATH) or os.path.getmtime(DRIVER_PATH) < max(
             os.path.getmtime(DRIVER_SRC), os.path.getmtime(DEFAULT_LIB_PATH)):
         build_driver()

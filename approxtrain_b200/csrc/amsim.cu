@@ -23,6 +23,12 @@
 #endif
 #include "amsim_kernels.cuh"
 #include "amsim_wide.cuh"
+#include "amsim_codes.cuh"
+#include "amsim_codes_launch.h"
+#include "amsim_factor.h"
+#ifndef AMSIM_SPLIT_TU
+#include "amsim_codes.cu"
+#endif
 
 #include <atomic>
 
@@ -69,6 +75,7 @@ struct Switches {
   int wide = -1;            // AMSIM_WIDE=0/1            wide-tile filter gradient: never / whenever eligible
   int capture_cluster = -1; // AMSIM_CAPTURE_CLUSTER=0/1 small launches inside a graph capture: balanced / cluster split
   int balanced_waves = -1;  // AMSIM_BALANCED_WAVES=n    CTAs of a balanced launch: n times the resident slots
+  int codes = -1;           // AMSIM_CODES=0/1           tensor-core path of factorable tables: never / whenever eligible
   int bounds_shrink = 0;    // AMSIM_BOUNDS_SHRINK=n     bounds-checking build only: the output's recorded extent is n bytes
                             //                           short, so its last stores are caught (self-test of the checker)
 };
@@ -96,6 +103,7 @@ void load_switches() {
   tri("AMSIM_WIDE", w.wide);
   tri("AMSIM_CAPTURE_CLUSTER", w.capture_cluster);
   tri("AMSIM_BALANCED_WAVES", w.balanced_waves);
+  tri("AMSIM_CODES", w.codes);
   tri("AMSIM_BOUNDS_SHRINK", w.bounds_shrink);
   g_sw = w;
 }
@@ -175,6 +183,9 @@ struct amsim_lut {
   uint8_t* d_canon = nullptr;  // encoded, row = first operand (a)   [m <= 7]
   uint8_t* d_trans = nullptr;  // encoded, row = second operand (b)  [m <= 7]
   int enc_bytes = 0;           // size of each encoded copy, multiple of 16
+  amsim::CodeTables codes;     // factorisation over 4-bit floats (slots == 0: none; the host copy holds no codes)
+  uint8_t* d_codes_f = nullptr;  // code rows of the first operand's indices [codes.slots / 2 bytes each]
+  uint8_t* d_codes_g = nullptr;  // ... and of the second operand's
   bool additive = false;       // encoded entry(i, j) == i + j for every pair: no lookups needed
   int direct = 0;              // LM_DIRECT_MBM / LM_DIRECT_MIT: no table at all, m = 23
   bool wide = false;           // 16-bit entries (d_raw / d_raw_t hold uint16), looked up in global memory
@@ -272,6 +283,18 @@ int upload_lut(const uint8_t* bytes, int m, int device, amsim_lut** out) {
     if (e == cudaSuccess) e = cudaMemcpy(h->d_canon, canon.data(), h->enc_bytes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(h->d_trans, trans.data(), h->enc_bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) bail(e, "upload of encoded lut");
+    if (rc == AMSIM_OK) {
+      h->codes = amsim::factor_table(canon.data(), m);
+      if (h->codes.slots) {
+        e = cudaMalloc(&h->d_codes_f, h->codes.f.size());
+        if (e == cudaSuccess) e = cudaMalloc(&h->d_codes_g, h->codes.g.size());
+        if (e == cudaSuccess) e = cudaMemcpy(h->d_codes_f, h->codes.f.data(), h->codes.f.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(h->d_codes_g, h->codes.g.data(), h->codes.g.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) bail(e, "upload of the table's codes");
+        h->codes.f = std::vector<uint8_t>();
+        h->codes.g = std::vector<uint8_t>();
+      }
+    }
   }
   if (rc == AMSIM_OK && m > 7) {
     const size_t side = (size_t)1 << m;
@@ -288,6 +311,8 @@ int upload_lut(const uint8_t* bytes, int m, int device, amsim_lut** out) {
     cudaFree(h->d_raw);
     cudaFree(h->d_canon);
     cudaFree(h->d_trans);
+    cudaFree(h->d_codes_f);
+    cudaFree(h->d_codes_g);
     delete h;
     return rc;
   }
@@ -338,6 +363,14 @@ void fill_lut(Params& p, const amsim_lut* lut, bool v_is_first_operand) {
   p.exact_only = sw().exact_only;
   uint32_t al = 16;
   while (al < (uint32_t)lut->enc_bytes) al <<= 1;
+  p.ct_slots = lut->codes.slots;
+  p.ct_unit = (float)lut->codes.unit;
+  p.ct_v = reinterpret_cast<const uint4*>(v_is_first_operand ? lut->d_codes_f : lut->d_codes_g);
+  p.ct_u = reinterpret_cast<const uint4*>(v_is_first_operand ? lut->d_codes_g : lut->d_codes_f);
+  p.ct_rows_v = v_is_first_operand ? lut->codes.rows_f : lut->codes.rows_g;
+  p.ct_rows_u = v_is_first_operand ? lut->codes.rows_g : lut->codes.rows_f;
+  p.ct_sh_v = 23 - lut->m + (v_is_first_operand ? lut->codes.drop_f : lut->codes.drop_g);
+  p.ct_sh_u = 23 - lut->m + (v_is_first_operand ? lut->codes.drop_g : lut->codes.drop_f);
   p.lut_align = al;  // m > 7: no table in shared memory (enc_bytes = 0)
 }
 
@@ -613,10 +646,135 @@ int launch_gather_t(cudaStream_t st, Params& p, int batch, int device) {
   CUDA_TRY(cudaLaunchKernelEx(&cfg, gather_gemm<1, EXACT, VEC, kClusterMode, LM>, p));
   return AMSIM_OK;
 }
+
+// ---- tensor-core path of factorable tables (amsim_codes.cuh) ------------------------------------
+// Set by a kernel whose bounded wait ran out (its results are wrong); read by amsim_debug_wait_report.
+__device__ unsigned g_code_stuck;
+
+int code_stuck_address(int device, unsigned** out) {
+  static std::mutex mu;
+  static std::map<int, unsigned*> known;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = known.find(device);
+  if (it == known.end()) {
+    void* p = nullptr;
+    CUDA_TRY(cudaGetSymbolAddress(&p, g_code_stuck));
+    it = known.emplace(device, static_cast<unsigned*>(p)).first;
+  }
+  *out = it->second;
+  return AMSIM_OK;
+}
+
+struct CodePlan {
+  int use = 0, shape = 0;
+  long long tiles = 0, iters = 0;
+  int grid = 0;
+  size_t slot_bytes = 0;     // parked tiles of the whole launch
+  size_t counter_bytes = 0;
+};
+
+// Whether and how the tensor-core path runs a P x Q x K problem.  Depends on the dimensions, the
+// device and the debug switches only, so that the *_workspace functions agree with the launch.
+CodePlan plan_codes(int P, int Q, int K, int batch, int sms) {
+  CodePlan f;
+  // a switch that picks among the table kernels keeps the launch on them
+  const Switches& w = sw();
+  const bool picked = w.balanced >= 0 || w.force_ksplit >= 0 || w.no_qsplit || w.no_uvec || w.no_wgrad_swap || w.thin_fast >= 0 || w.wide >= 0;
+  if (w.codes == 0 || (w.codes < 0 && picked) || P <= 0 || Q <= 0 || K <= 0 || batch <= 0) return f;
+  f.shape = Q > 128 ? 0 : Q > 64 ? 1 : 2;
+  const CodeTile t = code_tile(f.shape);
+  const long long pt = ((long long)P + t.bm - 1) / t.bm, qt = ((long long)Q + t.bn - 1) / t.bn;
+  f.tiles = pt * qt * batch;
+  f.iters = f.tiles * (((long long)K + CT_KB - 1) / CT_KB);
+  if ((long long)P + t.bm >= (1ll << 31) || (long long)K + CT_KB >= (1ll << 31)) return f;
+  // A launch of this kernel costs about 30 us more than one of the table kernels before it is at full rate
+  // (tables, tensor memory, tiles of 128 x 256): below 4e8 products, or with less than half of a tile's
+  // rows or columns used, it does not win that back.
+  if (sw().codes < 0 && ((double)P * Q * K * batch < 4e8 || P < 96 || Q < 48)) return f;
+  f.grid = (int)std::min<long long>(sms, std::max<long long>(1, f.iters / 2));
+  f.slot_bytes = (size_t)f.grid * 2 * t.slot_bytes;
+  f.counter_bytes = ((size_t)f.tiles * sizeof(int) + 255) / 256 * 256;
+  f.use = 1;
+  return f;
+}
+
+void code_params(CodeParams& c, const Params& p, const CodePlan& f, bool fgrad) {
+  const CodeTile t = code_tile(f.shape);
+  c.prm = p;
+  c.prm.sk_iters = f.iters;
+  c.prm.sk_ptiles = (p.P + t.bm - 1) / t.bm;
+  c.prm.sk_qtiles = (p.Q + t.bn - 1) / t.bn;
+  c.prm.sk_grid = f.grid;
+  c.tab_v = p.ct_v;
+  c.tab_u = p.ct_u;
+  c.rows_v = p.ct_rows_v;
+  c.rows_u = p.ct_rows_u;
+  c.sh_v = p.ct_sh_v;
+  c.sh_u = p.ct_sh_u;
+  c.unit = p.ct_unit;
+  c.fgrad = fgrad ? 1 : 0;
+  const bool va = aligned16(p.V) && p.v_bs % 4 == 0;
+  if (fgrad) c.v_mode = va && p.g.SC % 4 == 0 ? CT_RVEC : CT_RSCL;
+  else if (p.v_trans) c.v_mode = va && p.v_ld % 4 == 0 ? CT_RVEC : CT_RSCL;
+  else c.v_mode = va && p.g.SC % 4 == 0 ? CT_KVEC : CT_KSCL;
+  const bool ua = aligned16(p.U) && p.u_bs % 4 == 0 && p.u_tap % 4 == 0;
+  if (p.u_sq == 1) c.u_mode = ua && p.u_sk % 4 == 0 && p.Q % 4 == 0 ? CT_RVEC : CT_RSCL;
+  else if (p.u_sk == 1) c.u_mode = ua && p.u_sq % 4 == 0 && p.g.SC % 4 == 0 && !fgrad ? CT_KVEC : CT_KSCL;
+  else c.u_mode = CT_RSCL;
+  const long long lim = 1ll << 31;
+  c.step_v = !fgrad && c.v_mode == CT_KVEC && p.g.SC % CT_KB == 0 && p.v_elems < lim;
+  c.step_u = (c.u_mode == CT_RVEC || c.u_mode == CT_KVEC) && (fgrad ? p.K % CT_KB == 0 : p.g.SC % CT_KB == 0) &&
+             p.u_elems + (long long)CT_KB * p.u_sk < lim;
+}
+
+// counters: f.counter_bytes of zeros; parked: f.slot_bytes.
+int launch_codes(cudaStream_t st, const Params& p, const CodePlan& f, bool fgrad, void* counters, void* parked, int device) {
+  CodeParams c;
+  code_params(c, p, f, fgrad);
+  c.prm.ws = static_cast<float*>(parked);
+  c.prm.sk_count = static_cast<int*>(counters);
+  int rc = code_stuck_address(device, &c.stuck);
+  if (rc) return rc;
+  AMSIM_COUNT_LAUNCH();
+  CUDA_TRY(code_gemm_launch(st, c, f.shape, device));
+  return AMSIM_OK;
+}
+
+// 128-slot tables (all 7 bits of a mantissa matter, MIT_7) cost twice the codes per product: no faster than
+// the additive-table kernels, which need no lookups.
+bool codes_eligible(const Params& p, bool exact) {
+  return !exact && p.ct_slots > 0 && (p.ct_slots <= 64 || sw().codes > 0) && (p.lut_mode == LM_SMEM || p.lut_mode == LM_ADD);
+}
+
 int launch_gather(cudaStream_t st, Params& p, int batch, bool exact, int device) {
   if (p.P <= 0 || p.Q <= 0 || batch <= 0) return AMSIM_OK;  // nothing to compute
   fill_bounds(p, device, nullptr, 0);
   if ((long long)p.P >= (1ll << 31) - 256) return fail(AMSIM_ERR_UNSUPPORTED, "more than 2^31 output rows");
+  if (codes_eligible(p, exact)) {
+    const CodePlan f = plan_codes(p.P, p.Q, p.K, batch, sm_count(device));
+    if (f.use) {
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+      const size_t bytes = kPersistentCounterBytes + f.slot_bytes + f.counter_bytes;
+      BalancedScratch sc;
+      int rc = balanced_scratch_acquire(st, device, bytes, cap != cudaStreamCaptureStatusNone, &sc);
+      if (rc) return rc;
+      if (sc.ws) {
+        char* base = reinterpret_cast<char*>(sc.ws);
+        const bool clean = !sc.pooled && (size_t)f.tiles <= kPersistentCounters;
+        char* counters = clean ? base : base + kPersistentCounterBytes + f.slot_bytes;
+        Params q = p;
+        fill_bounds(q, device, base, bytes);
+        cudaError_t e1 = clean ? cudaSuccess : cudaMemsetAsync(counters, 0, f.counter_bytes, st);
+        rc = e1 == cudaSuccess ? launch_codes(st, q, f, false, counters, base + kPersistentCounterBytes, device) : AMSIM_OK;
+        const cudaError_t e2 = balanced_scratch_release(st, sc);
+        CUDA_TRY(e1);
+        if (rc) return rc;
+        CUDA_TRY(e2);
+        return AMSIM_OK;
+      }
+    }
+  }
   const bool vec = !p.v_trans && (p.g.SC % 4 == 0) && aligned16(p.V) && (p.v_bs % 4 == 0);
   // U by 128-bit loads along its contiguous index when four elements are always one aligned
   // group inside one tap: along q (weights of a forward convolution / dense layer / matmul B),
@@ -739,6 +897,8 @@ size_t fgrad_workspace(int P, int Q, int K, bool exact, int sms) {
         if (np) need = std::max(need, plan_fgrad(P, Q, K, false, np, sms).ws_bytes);
       }
     }
+    const CodePlan c = plan_codes(P, Q, K, 1, sms);
+    if (c.use) need = std::max(need, c.counter_bytes + c.slot_bytes);
   }
   return need;
 }
@@ -833,6 +993,16 @@ int launch_fgrad(cudaStream_t st, Params& p, bool exact, void* ws, size_t ws_byt
   if (p.P <= 0 || p.Q <= 0) return AMSIM_OK;
   if (lm_direct(p.lut_mode)) exact = true;  // one kernel flavour for the direct models: ordered chains
   const int sms = sm_count(device);
+  if (codes_eligible(p, exact)) {
+    // (a caller whose workspace does not hold the parked tiles takes the split-K kernels below)
+    const CodePlan c = plan_codes(p.P, p.Q, p.K, 1, sms);
+    if (c.use && ws && aligned16(ws) && ws_bytes >= c.counter_bytes + c.slot_bytes) {
+      Params q = p;
+      fill_bounds(q, device, ws, c.counter_bytes + c.slot_bytes);
+      CUDA_TRY(cudaMemsetAsync(ws, 0, c.counter_bytes, st));
+      return launch_codes(st, q, c, true, ws, static_cast<char*>(ws) + c.counter_bytes, device);
+    }
+  }
   const bool vec = (p.g.SC % 4 == 0) && aligned16(p.V);
   FgradPlan f = plan_fgrad(p.P, p.Q, p.K, exact, 0, sms);
   if (!exact && !f.thin && (p.lut_mode == LM_SMEM || p.lut_mode == LM_ADD)) {
@@ -962,6 +1132,18 @@ int amsim_debug_bounds_report(unsigned long long* word) {
 #endif
 }
 
+int amsim_debug_wait_report(unsigned* stuck) {
+  if (!stuck) return fail(AMSIM_ERR_INVALID, "NULL argument");
+  *stuck = 0;
+  unsigned* p = nullptr;
+  int rc = code_stuck_address(current_device(), &p);
+  if (rc) return rc;
+  CUDA_TRY(cudaDeviceSynchronize());
+  CUDA_TRY(cudaMemcpy(stuck, p, sizeof(*stuck), cudaMemcpyDeviceToHost));
+  CUDA_TRY(cudaMemset(p, 0, sizeof(*stuck)));
+  return AMSIM_OK;
+}
+
 void amsim_debug_reload_env(void) {
   sw();  // make sure the one-time load has happened, then replace its result
   load_switches();
@@ -1055,6 +1237,8 @@ int amsim_lut_close(amsim_lut* lut) {
   cudaFree(lut->d_raw_t);
   cudaFree(lut->d_canon);
   cudaFree(lut->d_trans);
+  cudaFree(lut->d_codes_f);
+  cudaFree(lut->d_codes_g);
   cudaSetDevice(prev);
   delete lut;
   return AMSIM_OK;

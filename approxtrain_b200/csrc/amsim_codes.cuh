@@ -1,0 +1,886 @@
+// Table GEMM on the tensor cores: the abstract product of amsim_kernels.cuh,
+//     Out[p, q] = sum_k AM(V[p, k], U[k, q]),
+// for tables that factor exactly over 4-bit floats.
+//
+// A product is  +-2^(ev + eu - 254) * T[iv][iu]  with T the table (values 1..4 in steps of
+// 2^-m).  When the table is opened the library looks for a factorisation
+//     T[i][j] = unit * sum_s F[i][s] * G[j][s],   s < S slots, all F and G in {0, .5, 1, 1.5, 2, 3, 4, 6, -...}
+// (factor_table in amsim.cu; every shipped table has one with S = its number of distinct rows:
+// row s + 1 minus row s is a handful of small integers).  A reduction step of the GEMM is then S
+// steps of a block-scaled 4-bit matrix product (tcgen05.mma kind::mxf4): an operand element
+// contributes a row of S codes looked up by its mantissa index (signs by flipping the codes' sign
+// bits), and its EXPONENT FIELD is the block's E8M0 scale byte as it stands.  The tensor core
+// forms sum_s F * G exactly (small integers times one power of two), so the product of every
+// element pair is the table's, and adds it to an FP32 accumulator in tensor memory.
+//
+// The accumulator add truncates (measured: one round toward zero per instruction, with at least 34
+// fraction bits kept before it), where an FP32 add rounds to nearest.  So every 128 reduction steps
+// the tile is added (round to nearest) to an FP32 partial tile in scratch and the tensor-memory tile
+// starts from zero: truncation errors never add up over more than 128 steps.  Measured against the
+// reference-order result the path is within 4e-8 (short reductions) to 3e-7 (10^5 steps), like the
+// split sums of the shared-memory kernels.
+//
+// Rates: 64 code steps of a 128 x 256 tile take 128 clocks (measured, also with all multiprocessors
+// busy), so 64-slot tables run at most 256 products per clock and multiprocessor, 8 times the 32
+// table lookups per clock that bound the shared-memory kernels.  What bounds this kernel is making
+// the operands: per reduction step and operand row S / 2 bytes of codes are looked up in a table,
+// sign-flipped and stored, all through the 128-byte/clock path to shared memory that the tensor
+// core reads from too (266 wavefronts per step of a 128 x 256 tile, 64-slot table).  Hence the codes
+// of V go to tensor memory instead (the product takes its first operand from there).
+//
+// One CTA per multiprocessor: 12 warps own 32 operand rows each (4 MT warps the rows of V, the rest
+// the columns of U): a warp fetches the raw FP32 elements of its rows with its own cp.async double
+// buffer, encodes them, and signals the stage; one more warp issues the matrix products.  No barrier
+// spans the CTA inside the loop.  Work is dealt out in equal runs of (tile, 16-step block) pairs as
+// in gather_gemm's balanced mode.
+//
+// Measured (MBM_7, B200): 3x3 256 -> 256 on 64 x 14 x 14, forward 1255 -> 318 us, filter gradient
+// 1250 -> 349 us (gather_gemm / wide_fgrad -> code_gemm).
+#pragma once
+#include "amsim_kernels.cuh"
+#include "amsim_wide.cuh"
+
+namespace amsim {
+
+constexpr int CT_KB = 16;        // reduction steps per block (one cp.async buffer of a warp)
+constexpr int CT_CHUNK = 8;      // blocks summed in tensor memory before they go to the FP32 partial tile
+constexpr int CT_MAXSPIN = 1 << 22;  // bound on every wait (a wait gives up, the kernel drains and reports)
+
+// How an operand's elements sit in memory.
+constexpr int CT_KVEC = 0;   // 16-byte groups of four consecutive reduction steps of one row
+constexpr int CT_RVEC = 1;   // 16-byte groups of four consecutive rows of one reduction step
+constexpr int CT_KSCL = 2;   // element by element, lanes along the reduction
+constexpr int CT_RSCL = 3;   // element by element, lanes along the rows
+
+struct CodeParams {
+  Params prm;
+  const uint4* tab_v;        // code rows of the lane operand's table indices (last row: zeros)
+  const uint4* tab_u;
+  int rows_v, rows_u;        // indices per table (the zero row is number rows_*)
+  int sh_v, sh_u;            // bits >> sh & (rows - 1) is the table index
+  float unit;                // out = acc * unit (a power of two)
+  int v_mode, u_mode;        // CT_* of the operands
+  int step_v, step_u;        // blocks never straddle a tap and offsets fit 32 bits: step through them
+  int fgrad;                 // V is gathered along p with the reduction over grid positions
+  unsigned* stuck;           // set when a bounded wait ran out
+};
+
+template <int S>
+struct CodeCfg {
+  static constexpr int KS = 256 / S;              // reduction steps per stage (a row of a stage is 128 bytes of codes)
+  static constexpr int CH = S / 32;               // 16-byte chunks per code row
+  static constexpr int W = S == 128 ? 1 : 2;      // scale words per row and stage
+  static constexpr int REP = S == 128 ? 4 : 8;    // copies of a code table: lanes of a quarter warp read different banks
+  static constexpr int STAGES_PER_KB = CT_KB / KS;
+};
+
+template <int S, int MT, int BN>
+struct CodeSmem {
+  using C = CodeCfg<S>;
+  static constexpr int BM = 128 * MT;
+  static constexpr int NW = 4 * MT + BN / 32;
+  static constexpr int NT = 32 * (NW + 1);
+  static constexpr int NBH = (BN + 127) / 128;    // 512-byte scale chunks of U per word
+  // stages in flight: a stage lives from the encoding of its rows to the end of its products (about
+  // 2000 clocks, of which the products take 512), so two stages leave the tensor core waiting
+  static constexpr int NST = MT == 2 && BN == 128 ? 3 : S == 128 ? 3 : 4;
+  static constexpr int CODE_BYTES = BN * 128;     // the codes of V go to tensor memory
+  static constexpr int SF_BYTES = (MT + NBH) * C::W * 512;
+  static constexpr int OFF_SF = NST * CODE_BYTES;
+  static constexpr int OFF_RAW = OFF_SF + NST * SF_BYTES;
+  // tensor memory columns: accumulators, NST stages of V codes, two sets of scales
+  static constexpr int T_CODES = MT * BN;
+  static constexpr int T_SF = T_CODES + NST * MT * 32;
+  static constexpr int SF_COLS = (MT + NBH) * C::W * 4;
+  static_assert(T_SF + 2 * SF_COLS <= 512, "tensor memory");
+  static constexpr int OFF_ROW = OFF_RAW + NW * 2 * 2048;
+  static constexpr int OFF_TAB = OFF_ROW + BM * 16;
+  static size_t bytes(int rows_v, int rows_u) {
+    return 1024 + OFF_TAB + (size_t)(rows_v + 1 + rows_u + 1) * C::CH * C::REP * 16;
+  }
+};
+
+// ---- tensor-core plumbing ---------------------------------------------------------------------
+__device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// Shared-memory matrix descriptor: layout 2 = rows of 128 bytes, 128-byte swizzle, 8-row groups 1024
+// bytes apart; layout 0 = 8 x 16-byte core matrices, 128 bytes apart (scale chunks).
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo, int layout) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46) |
+         ((uint64_t)layout << 61);
+}
+// kind::mxf4: E2M1 codes, E8M0 scales, FP32 accumulator; M = 128
+__host__ __device__ constexpr uint32_t code_idesc(int n) {
+  return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | (1u << 27);
+}
+__device__ __forceinline__ void mma_codes(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{.reg .pred p; setp.ne.b32 p, %6, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], %2, %3, [%4], [%5], p;}" ::"r"(d),
+      "r"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void scales_to_tmem(uint32_t taddr, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool elect_lane() {
+  uint32_t e;
+  asm volatile("{.reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p;}" : "=r"(e));
+  return e != 0;
+}
+__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint4 (&q)[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,"
+      "%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(q[0].x), "r"(q[0].y), "r"(q[0].z), "r"(q[0].w), "r"(q[1].x), "r"(q[1].y), "r"(q[1].z), "r"(q[1].w), "r"(q[2].x),
+      "r"(q[2].y), "r"(q[2].z), "r"(q[2].w), "r"(q[3].x), "r"(q[3].y), "r"(q[3].z), "r"(q[3].w), "r"(q[4].x), "r"(q[4].y),
+      "r"(q[4].z), "r"(q[4].w), "r"(q[5].x), "r"(q[5].y), "r"(q[5].z), "r"(q[5].w), "r"(q[6].x), "r"(q[6].y), "r"(q[6].z),
+      "r"(q[6].w), "r"(q[7].x), "r"(q[7].y), "r"(q[7].z), "r"(q[7].w)
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cp_async16n(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// Waits for a phase of an mbarrier, at most CT_MAXSPIN tries; after a wait has run out every later
+// one of this thread passes at once, so the kernel runs to its end (with wrong results) and reports.
+struct Waiter {
+  unsigned* stuck;
+  bool dead;
+  __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
+    if (dead) return;
+    for (int i = 0; i < CT_MAXSPIN; ++i)
+      if (mbar_try(bar, parity)) return;
+    dead = true;
+    atomicExch(stuck, 1u);
+  }
+  __device__ __forceinline__ void wait_warp(uint32_t bar, uint32_t parity) {
+    wait(bar, parity);
+    __syncwarp();
+  }
+};
+
+// Copies a code table to shared memory as [chunk][index][copy].
+template <int CH, int REP>
+__device__ __forceinline__ void copy_code_table(uint4* dst, const uint4* __restrict__ src, int rows, int tid, int nthreads) {
+  for (int i = tid; i < rows * CH * REP; i += nthreads) {
+    const int rest = i / REP, c = rest / rows, row = rest - c * rows;
+    dst[i] = __ldg(src + row * CH + c);
+  }
+}
+
+// Fetches the 32 rows x 16 reduction steps a warp encodes, raw FP32, into its 2 KB buffer:
+// CT_K*: row r at 64 r, its four 16-byte groups at (group ^ (r >> 1 & 3)); CT_R*: step k at 128 k.
+struct RowFetch {
+  int e_kh, e_kw, e_ch;  // filter tap of this lane's row (group) of a filter gradient
+  bool e_ok;
+  // Stepping (cp.step): where a block of 16 steps never straddles a filter tap, the four 16-byte groups a
+  // lane copies per block sit at offsets that advance by a constant until the tap ends.  (Decoding the tap and
+  // the rows anew for every block took as many instructions as encoding a stage.)
+  int off[4];            // element offsets of the next block's groups
+  int left;              // blocks left in the tap
+  uint32_t okm;          // bit i: group i exists
+
+  // r: first row of the warp inside the tile; for a new tile at (p0, q0)
+  __device__ __forceinline__ void new_tile(const CodeParams& cp, bool is_v, int first, int4* rowinfo, int lane) {
+    left = 0;
+    if (!is_v) return;
+    const Params& prm = cp.prm;
+    const Gather& g = prm.g;
+    if (cp.fgrad) {
+      const uint32_t pg = (uint32_t)(first + (cp.v_mode == CT_RVEC ? 4 * (lane & 7) : lane));
+      const uint32_t tap = fdiv(pg, g.d_sc);
+      e_ch = (int)(pg - tap * (uint32_t)g.SC);
+      e_kh = (int)fdiv(tap, g.d_kw);
+      e_kw = (int)tap - e_kh * g.KW;
+      e_ok = pg < (uint32_t)prm.P;
+      return;
+    }
+    const uint32_t pg = (uint32_t)(first + lane);
+    const uint32_t n = fdiv(pg, g.d_img);
+    const uint32_t rem = pg - n * (uint32_t)(g.PH * g.PW);
+    const uint32_t a = fdiv(rem, g.d_pw);
+    const uint32_t b = rem - a * (uint32_t)g.PW;
+    const long long nb = (long long)n * ((long long)g.SH * g.SW * g.SC);
+    int4 ri;
+    ri.x = pg < (uint32_t)prm.P ? (int)a * g.ps_h - g.off_t : INT32_MIN / 2;  // a row past the end is never in range
+    ri.y = (int)b * g.ps_w - g.off_l;
+    ri.z = (int)(uint32_t)nb;
+    ri.w = (int)(nb >> 32);
+    __syncwarp();
+    rowinfo[lane] = ri;
+    __syncwarp();
+  }
+
+  __device__ __forceinline__ void issue4(const Params& prm, int which, const float* __restrict__ base, int step, uint32_t dst,
+                                         uint32_t dst_step) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      bool ok = (okm >> i) & 1u;
+      const float* src = base + (ok ? off[i] : 0);
+      ok = ok && AMSIM_IN(prm, which, src, float4);
+      cp_async16n(dst + i * dst_step, src, ok ? 16 : 0);
+      off[i] += step;
+    }
+    --left;
+  }
+  // CT_KVEC patch rows: group i of a lane = row 8 i + lane / 4, steps 4 (lane % 4)...
+  __device__ __forceinline__ void step_v(const CodeParams& cp, const float* __restrict__ Vg, int kb, const int4* rowinfo,
+                                         uint32_t dst, int lane) {
+    const Params& prm = cp.prm;
+    const Gather& g = prm.g;
+    if (left == 0) {
+      const int k = kb * CT_KB;
+      const int tap = (int)fdiv((uint32_t)k, g.d_sc), ch = k - tap * g.SC;
+      const int kh = (int)fdiv((uint32_t)tap, g.d_kw), kw = tap - kh * g.KW;
+      left = (g.SC - ch) / CT_KB;
+      okm = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int4 ri = rowinfo[i * 8 + (lane >> 2)];
+        const int u = ri.x + kh, v = ri.y + kw;
+        if ((unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w) okm |= 1u << i;
+        off[i] = ri.z + (u * g.SW + v) * g.SC + ch + 4 * (lane & 3);
+      }
+    }
+    const int r = lane >> 2;
+    issue4(prm, BUF_V, Vg, CT_KB, dst + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4), 8 * 64);
+  }
+  // CT_RVEC: group i = step 4 i + lane / 8, rows 4 (lane % 8)...; CT_KVEC: as above
+  __device__ __forceinline__ void step_u(const CodeParams& cp, const float* __restrict__ Ug, int first, int kb, uint32_t dst,
+                                         int lane) {
+    const Params& prm = cp.prm;
+    const bool rvec = cp.u_mode == CT_RVEC;
+    if (left == 0) {
+      const int k = kb * CT_KB;
+      if (cp.fgrad) {
+        left = INT32_MAX;
+      } else {
+        const int tap = (int)fdiv((uint32_t)k, prm.g.d_sc);
+        left = (prm.g.SC - (k - tap * prm.g.SC)) / CT_KB;
+      }
+      const int base = (int)u_offset(cp, k);
+      okm = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int q = first + (rvec ? 4 * (lane & 7) : i * 8 + (lane >> 2));
+        if (q < prm.Q) okm |= 1u << i;
+        off[i] = base + (rvec ? (4 * i + (lane >> 3)) * prm.u_sk + q : q * prm.u_sq + 4 * (lane & 3));
+      }
+    }
+    if (rvec) {
+      issue4(prm, BUF_U, Ug, CT_KB * prm.u_sk, dst + lane * 16, 512);
+    } else {
+      const int r = lane >> 2;
+      issue4(prm, BUF_U, Ug, CT_KB, dst + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4), 8 * 64);
+    }
+  }
+
+  __device__ __forceinline__ void fetch_v(const CodeParams& cp, const float* __restrict__ Vg, int first, int kb,
+                                          const int4* rowinfo, uint32_t dst, int lane) const {
+    const Params& prm = cp.prm;
+    const Gather& g = prm.g;
+    if (cp.fgrad) {
+      if (cp.v_mode == CT_RVEC) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int kl = i * 4 + (lane >> 3), pix = kb * CT_KB + kl;
+          const uint32_t n = fdiv((uint32_t)pix, g.d_img);
+          const uint32_t rem = (uint32_t)pix - n * (uint32_t)(g.PH * g.PW);
+          const uint32_t a = fdiv(rem, g.d_pw);
+          const uint32_t b = rem - a * (uint32_t)g.PW;
+          const int u = (int)a * g.ps_h - g.off_t + e_kh, v = (int)b * g.ps_w - g.off_l + e_kw;
+          bool ok = e_ok && pix < prm.K && (unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w;
+          const float* src = ok ? Vg + ((long long)n * ((long long)g.SH * g.SW * g.SC) + ((long long)(u * g.SW + v) * g.SC + e_ch)) : Vg;
+          ok = ok && AMSIM_IN(prm, BUF_V, src, float4);
+          cp_async16n(dst + kl * 128 + (lane & 7) * 16, src, ok ? 16 : 0);
+        }
+      } else {
+#pragma unroll 4
+        for (int kl = 0; kl < CT_KB; ++kl) {
+          const int pix = kb * CT_KB + kl;
+          const uint32_t n = fdiv((uint32_t)pix, g.d_img);
+          const uint32_t rem = (uint32_t)pix - n * (uint32_t)(g.PH * g.PW);
+          const uint32_t a = fdiv(rem, g.d_pw);
+          const uint32_t b = rem - a * (uint32_t)g.PW;
+          const int u = (int)a * g.ps_h - g.off_t + e_kh, v = (int)b * g.ps_w - g.off_l + e_kw;
+          bool ok = e_ok && pix < prm.K && (unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w;
+          const float* src = ok ? Vg + ((long long)n * ((long long)g.SH * g.SW * g.SC) + ((long long)(u * g.SW + v) * g.SC + e_ch)) : Vg;
+          ok = ok && AMSIM_IN(prm, BUF_V, src, float);
+          cp_async4(dst + kl * 128 + lane * 4, src, ok);
+        }
+      }
+      return;
+    }
+    if (prm.v_trans) {  // V[p, k] at V[k * v_ld + p]
+      if (cp.v_mode == CT_RVEC) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int kl = i * 4 + (lane >> 3), k = kb * CT_KB + kl, p = first + 4 * (lane & 7);
+          bool ok = k < prm.K && p < prm.P;
+          const float* src = ok ? Vg + (long long)k * prm.v_ld + p : Vg;
+          ok = ok && AMSIM_IN(prm, BUF_V, src, float4);
+          cp_async16n(dst + kl * 128 + (lane & 7) * 16, src, ok ? 16 : 0);
+        }
+      } else {
+#pragma unroll 4
+        for (int kl = 0; kl < CT_KB; ++kl) {
+          const int k = kb * CT_KB + kl, p = first + lane;
+          bool ok = k < prm.K && p < prm.P;
+          const float* src = ok ? Vg + (long long)k * prm.v_ld + p : Vg;
+          ok = ok && AMSIM_IN(prm, BUF_V, src, float);
+          cp_async4(dst + kl * 128 + lane * 4, src, ok);
+        }
+      }
+      return;
+    }
+    const bool vec = cp.v_mode == CT_KVEC;
+    const int kl = vec ? 4 * (lane & 3) : (lane & 15), k = kb * CT_KB + kl;
+    const uint32_t tap = fdiv((uint32_t)k, g.d_sc);
+    const int ch = k - (int)tap * g.SC;
+    const int kh = (int)fdiv(tap, g.d_kw);
+    const int kw = (int)tap - kh * g.KW;
+    const bool k_ok = k < prm.K;
+    if (vec) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = i * 8 + (lane >> 2);
+        const int4 ri = rowinfo[r];
+        const int u = ri.x + kh, v = ri.y + kw;
+        bool ok = k_ok && (unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w;
+        const long long nb = ((long long)ri.w << 32) | (uint32_t)ri.z;
+        const float* src = ok ? Vg + nb + ((long long)(u * g.SW + v) * g.SC + ch) : Vg;
+        ok = ok && AMSIM_IN(prm, BUF_V, src, float4);
+        cp_async16n(dst + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4), src, ok ? 16 : 0);
+      }
+    } else {
+#pragma unroll 4
+      for (int i = 0; i < 16; ++i) {
+        const int r = i * 2 + (lane >> 4);
+        const int4 ri = rowinfo[r];
+        const int u = ri.x + kh, v = ri.y + kw;
+        bool ok = k_ok && (unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w;
+        const long long nb = ((long long)ri.w << 32) | (uint32_t)ri.z;
+        const float* src = ok ? Vg + nb + ((long long)(u * g.SW + v) * g.SC + ch) : Vg;
+        ok = ok && AMSIM_IN(prm, BUF_V, src, float);
+        cp_async4(dst + r * 64 + (((kl >> 2) ^ ((r >> 1) & 3)) << 4) + (kl & 3) * 4, src, ok);
+      }
+    }
+  }
+
+  // Element offset of U[k, q = 0] (see Params).
+  __device__ __forceinline__ static long long u_offset(const CodeParams& cp, int k) {
+    const Params& prm = cp.prm;
+    if (cp.fgrad) return (long long)k * prm.u_sk;
+    const Gather& g = prm.g;
+    const uint32_t tap = fdiv((uint32_t)k, g.d_sc);
+    const int kk = k - (int)tap * g.SC;
+    const int tj = (int)fdiv(tap, g.d_kw);
+    const int tp = prm.u_t0 + tj * prm.u_tj + ((int)tap - tj * g.KW) * prm.u_ti;
+    return (long long)tp * prm.u_tap + (long long)kk * prm.u_sk;
+  }
+
+  __device__ __forceinline__ void fetch_u(const CodeParams& cp, const float* __restrict__ Ug, int first, int kb, uint32_t dst,
+                                          int lane) const {
+    const Params& prm = cp.prm;
+    if (cp.u_mode == CT_RVEC) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int kl = i * 4 + (lane >> 3), k = kb * CT_KB + kl, q = first + 4 * (lane & 7);
+        bool ok = k < prm.K && q < prm.Q;
+        const float* src = ok ? Ug + u_offset(cp, k) + q : Ug;
+        ok = ok && AMSIM_IN(prm, BUF_U, src, float4);
+        cp_async16n(dst + kl * 128 + (lane & 7) * 16, src, ok ? 16 : 0);
+      }
+    } else if (cp.u_mode == CT_KVEC) {
+      const int k = kb * CT_KB + 4 * (lane & 3);
+      const float* col = Ug + u_offset(cp, k);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = i * 8 + (lane >> 2), q = first + r;
+        bool ok = k < prm.K && q < prm.Q;
+        const float* src = ok ? col + (long long)q * prm.u_sq : Ug;
+        ok = ok && AMSIM_IN(prm, BUF_U, src, float4);
+        cp_async16n(dst + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4), src, ok ? 16 : 0);
+      }
+    } else if (cp.u_mode == CT_KSCL) {
+      const int kl = lane & 15, k = kb * CT_KB + kl;
+      const float* col = Ug + u_offset(cp, k);
+#pragma unroll 4
+      for (int i = 0; i < 16; ++i) {
+        const int r = i * 2 + (lane >> 4), q = first + r;
+        bool ok = k < prm.K && q < prm.Q;
+        const float* src = ok ? col + (long long)q * prm.u_sq : Ug;
+        ok = ok && AMSIM_IN(prm, BUF_U, src, float);
+        cp_async4(dst + r * 64 + (((kl >> 2) ^ ((r >> 1) & 3)) << 4) + (kl & 3) * 4, src, ok);
+      }
+    } else {
+#pragma unroll 4
+      for (int kl = 0; kl < CT_KB; ++kl) {
+        const int k = kb * CT_KB + kl, q = first + lane;
+        bool ok = k < prm.K && q < prm.Q;
+        const float* src = ok ? Ug + u_offset(cp, k) + (long long)q * prm.u_sq : Ug;
+        ok = ok && AMSIM_IN(prm, BUF_U, src, float);
+        cp_async4(dst + kl * 128 + lane * 4, src, ok);
+      }
+    }
+  }
+};
+
+// Writes 4 consecutive columns of one output row through the epilogue (see store_out_tile).
+__device__ __forceinline__ void store_out4(const Params& prm, float* __restrict__ orow, int qg, float (&o)[4], bool vec_out) {
+  if (prm.bias != nullptr || prm.relu || prm.scale != nullptr || prm.has_alpha) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (prm.has_alpha) o[r] = __fmul_rn(o[r], prm.alpha);
+      if (prm.scale != nullptr && qg + r < prm.Q) o[r] = __fmul_rn(o[r], __ldg(prm.scale + qg + r));
+      if (prm.bias != nullptr && qg + r < prm.Q) o[r] = __fadd_rn(o[r], __ldg(prm.bias + qg + r));
+      if (prm.relu) o[r] = o[r] < 0.f ? 0.f : o[r];
+    }
+  }
+  if (vec_out && qg + 3 < prm.Q) {
+    if (AMSIM_IN(prm, BUF_O, orow + qg, float4)) *reinterpret_cast<float4*>(orow + qg) = make_float4(o[0], o[1], o[2], o[3]);
+  } else {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (qg + r < prm.Q && AMSIM_IN(prm, BUF_O, orow + (long long)(qg + r) * prm.o_sq, float)) orow[(long long)(qg + r) * prm.o_sq] = o[r];
+  }
+}
+
+// Share of a thread in draining and writing a tile: 16-column units u = g, g + NG, ... of the tile (g = warp / 4), of
+// the tile row 32 * (warp % 4) + lane of 128-row subtile u / (BN / 16).
+template <int S, int MT, int BN>
+struct CodeAcc {
+  static constexpr int NG = CodeSmem<S, MT, BN>::NW / 4;
+  static constexpr int UNITS = MT * BN / 16;
+  static constexpr int UPT = (UNITS + NG - 1) / NG;
+  static constexpr int NTE = NG * 128;                 // threads that drain
+  static constexpr int SLOT_FLOATS = UPT * 16 * NTE;   // one parked tile
+};
+
+template <int S, int MT, int BN>
+__global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __grid_constant__ CodeParams cp) {
+  using C = CodeCfg<S>;
+  using L = CodeSmem<S, MT, BN>;
+  using A = CodeAcc<S, MT, BN>;
+  constexpr int NW = L::NW, BM = L::BM, KS = C::KS, W = C::W, CH = C::CH, REP = C::REP, NST = L::NST;
+  constexpr int NG = A::NG, UPT = A::UPT;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  __shared__ uint64_t bars[2 * NST + 2];
+  __shared__ uint32_t tmem_holder;
+  __shared__ int flag_s;
+  const Params& prm = cp.prm;
+  const Gather& g = prm.g;
+  const uint32_t smem0 = (smem_addr(smem_raw) + 1023u) & ~1023u;
+  uint8_t* const smem = smem_raw + (smem0 - smem_addr(smem_raw));
+  const int t = threadIdx.x, lane = t & 31;
+  const int w = __shfl_sync(0xffffffffu, t >> 5, 0);
+  const uint32_t bar0 = smem_addr(bars);
+  const uint32_t bar_full = bar0, bar_empty = bar0 + 8 * NST, bar_done = bar0 + 16 * NST, bar_free = bar_done + 8;
+
+  if (t == 0) {
+    for (int i = 0; i < NST; ++i) {
+      mbar_init(bar_full + 8 * i, NW);
+      mbar_init(bar_empty + 8 * i, 1);
+    }
+    mbar_init(bar_done, 1);
+    mbar_init(bar_free, 4 * NG);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (w == NW) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_holder)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  uint4* const tab_v = reinterpret_cast<uint4*>(smem + L::OFF_TAB);
+  uint4* const tab_u = tab_v + (cp.rows_v + 1) * CH * REP;
+  copy_code_table<CH, REP>(tab_v, cp.tab_v, cp.rows_v + 1, t, L::NT);
+  copy_code_table<CH, REP>(tab_u, cp.tab_u, cp.rows_u + 1, t, L::NT);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_holder, 0);
+
+  const int nkb_all = (prm.K + CT_KB - 1) / CT_KB;
+  long long run_at = balanced_begin(blockIdx.x, prm.sk_iters, prm.sk_grid);
+  const long long run_end = balanced_begin((long long)blockIdx.x + 1, prm.sk_iters, prm.sk_grid);
+  auto decode_tile = [&](long long at, int& tp, int& tq, int& tz, int& kb0, int& kb1) {
+    const long long tile = at / nkb_all;
+    kb0 = (int)(at - tile * nkb_all);
+    kb1 = kb0 + (int)min((long long)(nkb_all - kb0), run_end - at);
+    tq = (int)(tile % prm.sk_qtiles);
+    const long long rest = tile / prm.sk_qtiles;
+    tp = (int)(rest % prm.sk_ptiles);
+    tz = (int)(rest / prm.sk_ptiles);
+  };
+  Waiter wt{cp.stuck, false};
+
+  if (w == NW) {
+    // ---- issue warp: moves the scales to tensor memory and issues the products --------------------
+    // The whole warp walks the loop on warp-uniform values and one elected lane issues, so descriptors
+    // and addresses stay in uniform registers (with a single-lane loop the moves into uniform registers
+    // took 1200 clocks per stage, more than twice its products).
+    const bool elected = elect_lane();
+    uint32_t b = 0, phase = 0, sfset = 0, chunk = 0;
+    const uint64_t desc_codes = smem_desc(smem0, 16, 1024, 2), desc_sf = smem_desc(smem0 + L::OFF_SF, 128, 128, 0);
+    while (run_at < run_end) {
+      int tp, tq, tz, kb0, kb1;
+      decode_tile(run_at, tp, tq, tz, kb0, kb1);
+      run_at += kb1 - kb0;
+      const int n = min(BN, (prm.Q - tq * BN + 31) / 32 * 32);
+      const int mts = min(MT, (prm.P - tp * BM + 127) / 128);
+      const uint32_t idesc = code_idesc(n);
+      for (int kb = kb0; kb < kb1; kb += CT_CHUNK, ++chunk) {
+        const int stages = (min(kb1, kb + CT_CHUNK) - kb) * C::STAGES_PER_KB;
+        wt.wait_warp(bar_free, (chunk & 1) ^ 1);
+        uint32_t accumulate = 0;
+#pragma unroll 1
+        for (int i = 0; i < stages; ++i) {
+          wt.wait_warp(bar_full + 8 * b, phase);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t bd = desc_codes + b * (L::CODE_BYTES >> 4), sfd = desc_sf + b * (L::SF_BYTES >> 4);
+          const uint32_t at = tmem + L::T_CODES + b * MT * 32;
+          const uint32_t sf_t = tmem + L::T_SF + sfset * L::SF_COLS;  // [V: mt][w], [U: w] scale columns
+          const uint32_t sfu_t = sf_t + MT * W * 4;
+          if (elected) {
+#pragma unroll
+            for (int j = 0; j < MT * W; ++j) scales_to_tmem(sf_t + 4 * j, sfd + 32 * j);
+#pragma unroll
+            for (int j = 0; j < W; ++j)
+#pragma unroll
+              for (int h = 0; h < L::NBH; ++h) scales_to_tmem(sfu_t + (j * L::NBH + h) * 4, sfd + 32 * (MT * W + h * W + j));
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+              if (mt >= mts) continue;
+#pragma unroll
+              for (int s = 0; s < 4; ++s) {  // 64 code steps each; their two scale bytes sit in half (id 0 / 2) of a word
+                const int word = S == 128 ? 0 : s >> 1, id = S == 128 ? (s >> 1) * 2 : (s & 1) * 2;
+                mma_codes(tmem + mt * BN, at + mt * 32 + 8 * s, bd + 2 * s, idesc | ((uint32_t)id << 4) | ((uint32_t)id << 29),
+                          sf_t + (mt * W + word) * 4, sfu_t + word * L::NBH * 4, s > 0 ? 1u : accumulate);
+              }
+            }
+            tc_commit(bar_empty + 8 * b);
+            if (i + 1 == stages) tc_commit(bar_done);
+          }
+          __syncwarp();
+          accumulate = 1;
+          sfset ^= 1;
+          if (++b == NST) {
+            b = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else {
+    // ---- operand warps: 32 rows of V (w < 4 MT) or columns of U each ----------------------------
+    const bool is_v = w < 4 * MT;
+    const int wu = w - 4 * MT;
+    const int row0 = is_v ? 32 * w : 32 * wu;
+    uint8_t* const raw = smem + L::OFF_RAW + w * 4096;
+    const uint32_t raw_s = smem0 + L::OFF_RAW + w * 4096;
+    int4* const rowinfo = reinterpret_cast<int4*>(smem + L::OFF_ROW) + (is_v ? row0 : 0);
+    const bool kmode = is_v ? (cp.v_mode == CT_KVEC || cp.v_mode == CT_KSCL) : (cp.u_mode == CT_KVEC || cp.u_mode == CT_KSCL);
+    const int rows = is_v ? cp.rows_v : cp.rows_u, sh = is_v ? cp.sh_v : cp.sh_u;
+    const uint32_t row_mask = (uint32_t)rows - 1u;
+    const uint8_t* const tab = reinterpret_cast<const uint8_t*>((is_v ? tab_v : tab_u) + (lane & (REP - 1)));
+    const int tab_chunk = (rows + 1) * REP * 16;
+    // this lane's row in a code stage and its place among the scale words
+    const uint32_t code_t = tmem + L::T_CODES + (w >> 2) * 32 + ((uint32_t)(w & 3) << 21);
+    const uint32_t sf_off = L::OFF_SF + (is_v ? (w >> 2) * W * 512 : (MT + (wu >> 2)) * W * 512) + lane * 16 + ((is_v ? w : wu) & 3) * 4;
+
+    RowFetch rf;
+    long long ld_at = run_at;
+    int ld_p = 0, ld_q = 0, ld_z = 0, ld_kb = 0, ld_kb1 = 0, ld_buf = 0;
+    auto fetch_next = [&]() {
+      if (ld_kb == ld_kb1 && ld_at < run_end) {
+        decode_tile(ld_at, ld_p, ld_q, ld_z, ld_kb, ld_kb1);
+        ld_at += ld_kb1 - ld_kb;
+        rf.new_tile(cp, is_v, ld_p * BM + row0, rowinfo, lane);
+      }
+      if (ld_kb < ld_kb1) {
+        if (is_v) {
+          if (ld_p * BM + row0 >= prm.P) {
+          } else if (cp.step_v)
+            rf.step_v(cp, prm.V + (long long)ld_z * prm.v_bs, ld_kb, rowinfo, raw_s + ld_buf * 2048, lane);
+          else
+            rf.fetch_v(cp, prm.V + (long long)ld_z * prm.v_bs, ld_p * BM + row0, ld_kb, rowinfo, raw_s + ld_buf * 2048, lane);
+        } else if (ld_q * BN + row0 < prm.Q) {
+          if (cp.step_u)
+            rf.step_u(cp, prm.U + (long long)ld_z * prm.u_bs, ld_q * BN + row0, ld_kb, raw_s + ld_buf * 2048, lane);
+          else
+            rf.fetch_u(cp, prm.U + (long long)ld_z * prm.u_bs, ld_q * BN + row0, ld_kb, raw_s + ld_buf * 2048, lane);
+        }
+        ++ld_kb;
+        ld_buf ^= 1;
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    // Ring position: with a whole number of turns per block the stage buffer and its barriers are constants of
+    // the unrolled loop; otherwise they are counted.
+    constexpr int SPK = C::STAGES_PER_KB;
+    constexpr bool FIXED = SPK % NST == 0;
+    uint32_t b_var = 0, phase = 1, chunk = 0;  // stage buffer (not FIXED), parity of its 'empty' barrier
+    const uint32_t code_base = smem0 + (row0 + lane) * 128;
+    uint32_t code_sw[8];                       // this lane's eight 16-byte places in a stage row (128-byte swizzle)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) code_sw[i] = ((uint32_t)i << 4) ^ ((uint32_t)(lane & 7) << 4);
+    const int grp = w >> 2;
+    float* slot = nullptr;  // this thread's place among the parked tiles
+    // One unit of the finished tensor-memory tile plus what earlier chunks of the segment left in the slot.
+    auto load_unit = [&](int i, bool first, float (&v)[16]) {
+      uint32_t r[16];
+      tmem_load16(tmem + ((uint32_t)(w & 3) << 21) + (grp + i * NG) * 16, r);
+#pragma unroll
+      for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(r[c]);
+      if (!first) {
+#pragma unroll
+        for (int c = 0; c < 16; ++c)
+          if (AMSIM_IN(prm, BUF_WS, slot + (i * 16 + c) * A::NTE, float)) v[c] = __fadd_rn(__ldcg(slot + (i * 16 + c) * A::NTE), v[c]);
+      }
+    };
+    auto park_unit = [&](int i, const float (&v)[16]) {
+#pragma unroll
+      for (int c = 0; c < 16; ++c)
+        if (AMSIM_IN(prm, BUF_WS, slot + (i * 16 + c) * A::NTE, float)) __stcg(slot + (i * 16 + c) * A::NTE, v[c]);
+    };
+    auto begin_drain = [&]() {
+      wt.wait_warp(bar_done, chunk & 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    };
+    auto end_drain = [&]() {
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_free);
+    };
+    // Moves a finished chunk of the segment from tensor memory to the slot and frees it.
+    auto drain = [&](bool first) {
+      if (grp < NG) {
+        begin_drain();
+#pragma unroll 1
+        for (int i = 0; i < UPT; ++i) {
+          if (grp + i * NG >= A::UNITS) break;
+          float v[16];
+          load_unit(i, first, v);
+          park_unit(i, v);
+        }
+        end_drain();
+      }
+      ++chunk;
+    };
+
+    int buf = 0;
+    fetch_next();
+    while (run_at < run_end) {
+      int cp_, cq, cz, kb0, kb1;
+      decode_tile(run_at, cp_, cq, cz, kb0, kb1);
+      run_at += kb1 - kb0;
+      const bool active = is_v ? cp_ * BM + row0 < prm.P : cq * BN + row0 < prm.Q;
+      slot = prm.ws + ((long long)blockIdx.x * 2 + (kb0 == 0 ? 1 : 0)) * A::SLOT_FLOATS + t;
+      bool pending = false, fresh = true;
+      int since = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        fetch_next();
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const uint8_t* rb = raw + buf * 2048;
+        buf ^= 1;
+#pragma unroll
+        for (int j = 0; j < SPK; ++j) {
+          if (j == NST % SPK && pending && since == NST - NST % SPK) {  // the next chunk's first stages are made while the last one finishes
+            drain(fresh);
+            fresh = pending = false;
+          }
+          const uint32_t b = FIXED ? (uint32_t)(j % NST) : b_var;
+          uint32_t x[KS];
+          uint4 q[8];
+          if (active) {
+            if (kmode) {
+              if (KS == 2) {
+                const uint2 v = *reinterpret_cast<const uint2*>(rb + lane * 64 + (((j >> 1) ^ ((lane >> 1) & 3)) << 4) + (j & 1) * 8);
+                x[0] = v.x; x[1] = v.y;
+              } else {
+#pragma unroll
+                for (int i = 0; i < KS / 4; ++i) {
+                  const uint4 v = *reinterpret_cast<const uint4*>(rb + lane * 64 + (((j * (KS / 4) + i) ^ ((lane >> 1) & 3)) << 4));
+                  x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[(4 * i + 3) % KS] = v.w;
+                }
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < KS; ++i) x[i] = *reinterpret_cast<const uint32_t*>(rb + (j * KS + i) * 128 + lane * 4);
+            }
+            // all eight 16-byte pieces are read before the first is stored (the compiler cannot tell that the
+            // stage and the table do not overlap), and before the wait for the stage
+#pragma unroll
+            for (int e = 0; e < KS; ++e) {
+              // zero and denormal elements take the table's zero row: their products are exactly 0
+              const uint32_t idx = (x[e] & 0x7F800000u) ? ((x[e] >> sh) & row_mask) : (uint32_t)rows;
+              const uint8_t* src = tab + idx * (REP * 16);
+#pragma unroll
+              for (int c = 0; c < CH; ++c) q[e * CH + c] = *reinterpret_cast<const uint4*>(src + c * tab_chunk);
+            }
+          }
+          wt.wait_warp(bar_empty + 8 * b, phase);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (active) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint32_t sign = (uint32_t)((int)x[i / CH] >> 31) & 0x88888888u;
+              q[i].x ^= sign; q[i].y ^= sign; q[i].z ^= sign; q[i].w ^= sign;
+            }
+            if (is_v) {
+              tmem_store32(code_t + b * MT * 32, q);
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) sts128(code_base + code_sw[i] + b * L::CODE_BYTES, q[i]);
+            }
+            // scale bytes = exponent fields; one 32-bit word covers two matrix instructions
+            uint8_t* const sfp = smem + sf_off + b * L::SF_BYTES;
+            if (S == 64) {
+              *reinterpret_cast<uint32_t*>(sfp) = __byte_perm(x[0] << 1, x[1] << 1, 0x7733);
+              *reinterpret_cast<uint32_t*>(sfp + 512) = __byte_perm(x[2 % KS] << 1, x[3 % KS] << 1, 0x7733);
+            } else if (S == 128) {
+              *reinterpret_cast<uint32_t*>(sfp) = __byte_perm(x[0] << 1, x[1] << 1, 0x7733);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 2; ++i) {
+                const uint32_t lo = __byte_perm(x[(4 * i) % KS] << 1, x[(4 * i + 1) % KS] << 1, 0x0073);
+                const uint32_t hi = __byte_perm(x[(4 * i + 2) % KS] << 1, x[(4 * i + 3) % KS] << 1, 0x0073);
+                *reinterpret_cast<uint32_t*>(sfp + 512 * i) = __byte_perm(lo, hi, 0x5410);
+              }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_full + 8 * b);
+          if (FIXED) {
+            if ((j + 1) % NST == 0) phase ^= 1;
+          } else if (++b_var == NST) {
+            b_var = 0;
+            phase ^= 1;
+          }
+        }
+        since += SPK;
+        if ((kb - kb0 + 1) % CT_CHUNK == 0 && kb + 1 < kb1) {
+          pending = true;
+          since = 0;
+        }
+      }
+      if (pending) {
+        drain(fresh);
+        fresh = false;
+      }
+
+      // ---- epilogue: the last chunk and the slot make the segment's sums ---------------------------
+      if (grp < NG) {
+        const long long tile = ((long long)cz * prm.sk_ptiles + cp_) * prm.sk_qtiles + cq;
+        const bool shared_tile = kb0 != 0 || kb1 != nkb_all;
+        float* __restrict__ Og = prm.O + (long long)cz * prm.o_bs;
+        const bool vec_out = prm.o_sq == 1 && (prm.o_sp & 3) == 0 && (prm.o_bs & 3) == 0 && ((reinterpret_cast<uintptr_t>(prm.O) & 15) == 0);
+        auto write_unit = [&](int i, float (&v)[16]) {
+          const int u = grp + i * NG;
+          const int pg = cp_ * BM + (u / (BN / 16)) * 128 + (w & 3) * 32 + lane, q0 = cq * BN + (u % (BN / 16)) * 16;
+          if (pg >= prm.P || q0 >= prm.Q) return;
+          long long row = pg;
+          if (prm.o_strided) {
+            const uint32_t n = fdiv((uint32_t)pg, g.d_img);
+            const uint32_t rem = (uint32_t)pg - n * (uint32_t)(g.PH * g.PW);
+            const uint32_t yy = fdiv(rem, g.d_pw);
+            const uint32_t xx = rem - yy * (uint32_t)g.PW;
+            row = ((long long)n * prm.o_h + (long long)yy * prm.o_sh + prm.o_a) * prm.o_w + (long long)xx * prm.o_sw + prm.o_b;
+          }
+          float* orow = Og + row * prm.o_sp;
+#pragma unroll
+          for (int c4 = 0; c4 < 4; ++c4) {
+            float o[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) o[r] = __fmul_rn(v[4 * c4 + r], cp.unit);
+            store_out4(prm, orow, q0 + 4 * c4, o, vec_out);
+          }
+        };
+        begin_drain();
+#pragma unroll 1
+        for (int i = 0; i < UPT; ++i) {
+          if (grp + i * NG >= A::UNITS) break;
+          float v[16];
+          load_unit(i, fresh, v);
+          if (shared_tile) park_unit(i, v);
+          else write_unit(i, v);
+        }
+        end_drain();
+        if (shared_tile) {
+          // a tile shared between runs: count in; the last sharer adds the parked tiles in CTA order
+          __threadfence();
+          asm volatile("bar.sync 1, %0;" ::"r"(A::NTE) : "memory");
+          const long long first = tile * nkb_all, last = first + nkb_all;
+          long long c0 = first * prm.sk_grid / prm.sk_iters;
+          while (c0 > 0 && balanced_begin(c0, prm.sk_iters, prm.sk_grid) > first) --c0;
+          while (balanced_begin(c0 + 1, prm.sk_iters, prm.sk_grid) <= first) ++c0;
+          long long c1 = (last - 1) * prm.sk_grid / prm.sk_iters;
+          while (c1 > 0 && balanced_begin(c1, prm.sk_iters, prm.sk_grid) > last - 1) --c1;
+          while (balanced_begin(c1 + 1, prm.sk_iters, prm.sk_grid) <= last - 1) ++c1;
+          if (t == 0) {
+            const int arrived = AMSIM_IN(prm, BUF_WS, prm.sk_count + tile, int) ? atomicAdd(prm.sk_count + tile, 1) : 0;
+            flag_s = arrived == (int)(c1 - c0);
+            if (arrived == (int)(c1 - c0) && AMSIM_IN(prm, BUF_WS, prm.sk_count + tile, int)) prm.sk_count[tile] = 0;
+          }
+          asm volatile("bar.sync 1, %0;" ::"r"(A::NTE) : "memory");
+          const bool completes = flag_s != 0;
+          asm volatile("bar.sync 1, %0;" ::"r"(A::NTE) : "memory");
+          if (completes) {
+            __threadfence();
+#pragma unroll 1
+            for (int i = 0; i < UPT; ++i) {
+              if (grp + i * NG >= A::UNITS) break;
+              float v[16];
+#pragma unroll
+              for (int c = 0; c < 16; ++c) v[c] = 0.f;
+              for (long long cta = c0; cta <= c1; ++cta) {
+                const long long bg = balanced_begin(cta, prm.sk_iters, prm.sk_grid);
+                const float* src = prm.ws + (cta * 2 + (bg <= first ? 1 : 0)) * A::SLOT_FLOATS + t;
+#pragma unroll
+                for (int c = 0; c < 16; ++c)
+                  if (AMSIM_IN(prm, BUF_WS, src + (i * 16 + c) * A::NTE, float)) v[c] = __fadd_rn(v[c], __ldcg(src + (i * 16 + c) * A::NTE));
+              }
+              write_unit(i, v);
+            }
+          }
+        }
+      }
+      ++chunk;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (w == NW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
+}  // namespace amsim

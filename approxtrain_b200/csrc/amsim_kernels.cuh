@@ -126,7 +126,7 @@ struct Bounds {
   const char* hi[4];
   unsigned long long* report;  // 0 = clean; else line << 44 | (buffer + 1) << 40 | low 40 bits of the byte offset
 };
-__device__ __noinline__ void amsim_bounds_record(const Bounds& b, int which, const void* p, int line) {
+static __device__ __noinline__ void amsim_bounds_record(const Bounds& b, int which, const void* p, int line) {
   const unsigned long long off = (unsigned long long)((const char*)p - b.lo[which]) & ((1ull << 40) - 1);
   atomicCAS(b.report, 0ull, ((unsigned long long)line << 44) | ((unsigned long long)(which + 1) << 40) | off);
 }
@@ -197,6 +197,11 @@ struct Params {
   int sk_ptiles, sk_qtiles;     // tile grid (q runs fastest, then p, then batch)
   int sk_grid;                  // CTAs of the balanced launch
   int* sk_count;                // per tile: CTAs that have parked their share (zero before the launch)
+  // code_gemm (amsim_codes.cuh): the table's factorisation over 4-bit floats (0 slots: it has none)
+  int ct_slots, ct_rows_v, ct_rows_u, ct_sh_v, ct_sh_u;
+  float ct_unit;
+  const uint4* ct_v;
+  const uint4* ct_u;
   long long v_elems, u_elems, o_elems;  // extents of V, U and O in elements (bounds-checking build)
 #ifdef AMSIM_BOUNDS_CHECK
   Bounds bnd;
@@ -1419,6 +1424,7 @@ __global__ void __launch_bounds__(768) fgrad_exact_chain(const Params prm) {
     prm.O[(long long)pg * prm.o_sp + (long long)qg * prm.o_sq] = acc;
 }
 
+#ifndef AMSIM_TEMPLATES_ONLY  // kernels that are no templates: compiled with amsim.cu only
 // Sums the split-K partials in a fixed order (the result does not depend on scheduling).
 // Partials are [split][n]; the sum of element i goes to out[(i / Q) * o_sp + (i % Q) * o_sq].
 // `lanes` threads share one element: lane l adds the consecutive splits [l * per, (l + 1) * per)
@@ -1602,5 +1608,7 @@ __global__ void mul_elementwise(const float* __restrict__ a, const float* __rest
     out[i] = __uint_as_float(r);
   }
 }
+
+#endif  // AMSIM_TEMPLATES_ONLY
 
 }  // namespace amsim

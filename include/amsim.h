@@ -301,6 +301,12 @@ void amsim_debug_reload_env(void);
  * AMSIM_ERR_UNSUPPORTED and *word = 0.  No reference counterpart. */
 int amsim_debug_bounds_report(unsigned long long* word);
 
+/* The tensor-core kernels bound every wait between their warps; one that runs out makes the kernel
+ * end with wrong results instead of hanging.  This call waits for the device, returns nonzero in
+ * *stuck if that has happened on the current device since the last call (it never should), and clears
+ * the mark.  No reference counterpart. */
+int amsim_debug_wait_report(unsigned* stuck);
+
 /* Host-side check of the kernels' constant-divisor arithmetic (no GPU work):
  * returns n / d computed the way the device code does.  For tests. */
 uint32_t amsim_debug_fastdiv(uint32_t n, uint32_t d);

@@ -1,0 +1,99 @@
+"""The tensor-core path of factorable tables (code_gemm, AMSIM_CODES=1 forces it at any size) against
+deterministic mode, which is bit-identical to the reference: every table factorisation (32, 64 and 128
+slots), every operand layout the kernel fetches, and the sizes where its tiles and stages end.
+
+Bound: products are exact; a partial sum of at most 128 steps is truncated once per step, so it is off
+by at most 128 * 2^-23 of the partial sums' largest value (1.5e-5, if every step lost a whole bit), and
+about 2^-24 * sqrt(steps) on data whose products spread over many exponents: 1e-5 as for every fast kernel."""
+import ctypes as C
+import os
+
+import numpy as np
+import pytest
+
+from conftest import lut_path, rel_l2
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def forced(monkeypatch):
+    from approxtrain_b200 import _lib
+    monkeypatch.setenv("AMSIM_CODES", "1")
+    _lib.lib.amsim_debug_reload_env()
+    yield _lib
+    stuck = C.c_uint(1)
+    assert _lib.lib.amsim_debug_wait_report(C.byref(stuck)) == 0 and stuck.value == 0, "a wait between warps ran out"
+    monkeypatch.undo()
+    _lib.lib.amsim_debug_reload_env()
+
+
+def _close(got, want):
+    assert rel_l2(got.cpu().numpy(), want.cpu().numpy()) <= 1e-5
+
+
+# (n, h, w, c, kh, kw, k, stride, padding): tile edges in pixels and channels (k 64 / 65 / 128 / 129 / 257), taps that
+# end inside a 16-step block (c 8, 24, 37), reductions of one block, of more than one 128-step chunk, strides
+SHAPES = [(1, 16, 16, 16, 1, 1, 64, 1, "VALID"), (2, 9, 13, 16, 3, 3, 65, 1, "SAME"), (1, 16, 16, 24, 3, 3, 128, 1, "SAME"),
+          (3, 11, 7, 8, 3, 3, 129, 2, "SAME"), (2, 12, 12, 37, 5, 5, 257, 1, "SAME"), (1, 30, 30, 3, 7, 7, 64, 2, "VALID"),
+          (2, 14, 14, 256, 1, 1, 300, 1, "VALID"), (4, 20, 20, 64, 3, 3, 32, 1, "SAME")]
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7", "MIT_5", "ACC_7", "MBM_1"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_convolutions(forced, lut, shape):
+    from approxtrain_b200 import ops
+    n, h, w, c, kh, kw, k, s, pad = shape
+    g = torch.Generator(device="cuda").manual_seed(n * h + k)
+    x = torch.relu(torch.randn(n, h, w, c, generator=g, device="cuda"))
+    wt = torch.randn(kh, kw, c, k, generator=g, device="cuda")
+    kw_ = dict(strides=s, padding=pad, mant_mul_lut=lut_path(lut))
+    y = ops.convam(x, wt, **kw_)
+    _close(y, ops.convam(x, wt, deterministic=True, **kw_))
+    assert torch.equal(y, ops.convam(x, wt, **kw_)), "run-to-run identical"
+    dy = torch.randn(y.shape, generator=g, device="cuda")
+    _close(ops.convam_input_grad(x.shape, wt, dy, **kw_), ops.convam_input_grad(x.shape, wt, dy, deterministic=True, **kw_))
+    dw = ops.convam_filter_grad(wt.shape, x, dy, **kw_)
+    _close(dw, ops.convam_filter_grad(wt.shape, x, dy, deterministic=True, **kw_))
+    assert torch.equal(dw, ops.convam_filter_grad(wt.shape, x, dy, **kw_)), "run-to-run identical"
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7", "MBM_5"])
+@pytest.mark.parametrize("m,k,n,ta,tb", [(128, 64, 128, 0, 1), (100, 70, 90, 1, 0), (33, 129, 257, 1, 1), (128, 128, 64, 0, 0), (1, 5, 1, 0, 0)])
+def test_matmuls(forced, lut, m, k, n, ta, tb):
+    from approxtrain_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    a = torch.randn(*((3, k, m) if ta else (3, m, k)), generator=g, device="cuda")
+    b = torch.randn(*((3, n, k) if tb else (3, k, n)), generator=g, device="cuda")
+    f = lambda det: ops.matmulam(a, b, transpose_a=bool(ta), transpose_b=bool(tb), mant_mul_lut=lut_path(lut),  # noqa: E731
+                                 deterministic=det, alpha=0.125)
+    _close(f(False), f(True))
+
+
+def test_zeros_give_zero_and_non_finite_values_stay_visible(forced):
+    from approxtrain_b200 import ops
+    p = lut_path("MBM_7")
+    x = torch.zeros(200, 64, device="cuda")
+    w = torch.randn(64, 96, device="cuda")
+    assert torch.equal(ops.denseam(x, w, p), torch.zeros(200, 96, device="cuda"))
+    x[7, 3] = float("nan")
+    y = ops.denseam(x, w, p)
+    assert not torch.isfinite(y[7]).any() and torch.equal(y[:7], torch.zeros(7, 96, device="cuda"))
+
+
+def test_every_shipped_table_takes_the_path(forced):
+    """With AMSIM_CODES=0 the table kernels run: another order of the same sum, so the bits differ."""
+    from approxtrain_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, w = torch.randn(256, 300, generator=g, device="cuda"), torch.randn(300, 256, generator=g, device="cuda")
+    for lut in ("ACC_7", "MBM_3", "MBM_5", "MBM_7", "MIT_3", "MIT_5", "MIT_7"):
+        os.environ["AMSIM_CODES"] = "1"
+        forced.lib.amsim_debug_reload_env()
+        a = ops.denseam(x, w, lut_path(lut))
+        os.environ["AMSIM_CODES"] = "0"
+        forced.lib.amsim_debug_reload_env()
+        b = ops.denseam(x, w, lut_path(lut))
+        assert not torch.equal(a, b), lut
+        assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5
+    assert np.isfinite(a.cpu().numpy()).all()
