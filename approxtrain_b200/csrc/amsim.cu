@@ -31,6 +31,7 @@
 #endif
 
 #include <atomic>
+#include <cmath>
 
 // Kernels launched by this library since it was loaded (amsim_debug_launch_count).
 static std::atomic<unsigned long long> g_launches{0};
@@ -668,32 +669,63 @@ int code_stuck_address(int device, unsigned** out) {
 struct CodePlan {
   int use = 0, shape = 0;
   long long tiles = 0, iters = 0;
-  int grid = 0;
+  int grid = 0;              // CTA pairs
   size_t slot_bytes = 0;     // parked tiles of the whole launch
   size_t counter_bytes = 0;
 };
 
-// Whether and how the tensor-core path runs a P x Q x K problem.  Depends on the dimensions, the
-// device and the debug switches only, so that the *_workspace functions agree with the launch.
-CodePlan plan_codes(int P, int Q, int K, int batch, int sms) {
+// What the choice between the tensor-core path and the table kernels looks at besides the dimensions.
+struct CodeTraits {
+  int slots;           // of the table's factorisation
+  bool additive;       // the other path needs no lookups
+  bool fgrad, scalar;  // a filter gradient; operands that are fetched element by element
+};
+// The traits for which the path is taken most readily: the *_workspace functions do not know the table.
+constexpr CodeTraits kCodeTraitsAny = {32, false, true, false};
+
+// Microseconds of one launch on either path, fitted to 75 timed launches (1e6 to 9e9 products, MBM_7, MIT_7 and
+// MIT_5, B200).  Tensor cores: a fixed part, the 16-step blocks of one CTA pair (2.6 / 1.8 / 1.45 us for 256 / 128 /
+// 64 columns and 64 slots), and the parked tiles that the last pair to finish a shared tile adds up.  Table kernels:
+// 165 us per 1e9 lookups, 105 us per 1e9 additive products, and a part that long reductions over few tiles add.
+// Examples (table kernels / this path): 8192 x 512 x 128, MBM_7 110 / 47 us, MIT_7 78 / 70 us; 784 x 1152 x 128,
+// MBM_7 72 / 51 us; 1024 x 512 x 256, MIT_7 39 / 59 us.
+constexpr double kCodeBlockUs[3] = {2.6, 1.8, 1.45}, kCodeShareUs[3] = {2.2, 1.7, 1.0};
+double code_us(const CodePlan& f, const CodeTraits& t) {
+  const double block = kCodeBlockUs[f.shape] * (t.slots == 128 ? 1.9 : t.slots == 32 ? 0.85 : 1.0) * (t.scalar ? 1.4 : 1.0);
+  return 16 + ((double)f.iters / f.grid + 2) * block + ((double)f.grid / f.tiles + 1) * kCodeShareUs[f.shape];
+}
+double table_us(double products, int K, const CodeTraits& t) {
+  const double wide = (t.additive ? 24 + 105e-9 * products : 22 + 165e-9 * products) * (t.scalar ? 1.2 : 1.0);
+  return wide + (t.fgrad ? 0 : std::min(45.0, (t.additive ? 0.019 : 0.022) * std::max(0, K - 512)));
+}
+
+// Whether and how the tensor-core path runs a P x Q x K problem.  The grid depends on the dimensions, the device and
+// the debug switches only, so that a workspace sized for kCodeTraitsAny fits every launch.
+CodePlan plan_codes(int P, int Q, int K, int batch, int sms, const CodeTraits& t) {
   CodePlan f;
   // a switch that picks among the table kernels keeps the launch on them
   const Switches& w = sw();
   const bool picked = w.balanced >= 0 || w.force_ksplit >= 0 || w.no_qsplit || w.no_uvec || w.no_wgrad_swap || w.thin_fast >= 0 || w.wide >= 0;
   if (w.codes == 0 || (w.codes < 0 && picked) || P <= 0 || Q <= 0 || K <= 0 || batch <= 0) return f;
   f.shape = Q > 128 ? 0 : Q > 64 ? 1 : 2;
-  const CodeTile t = code_tile(f.shape);
-  const long long pt = ((long long)P + t.bm - 1) / t.bm, qt = ((long long)Q + t.bn - 1) / t.bn;
+  const CodeTile tile = code_tile(f.shape);
+  const long long pt = ((long long)P + tile.bm - 1) / tile.bm, qt = ((long long)Q + tile.bn - 1) / tile.bn;
   f.tiles = pt * qt * batch;
   f.iters = f.tiles * (((long long)K + CT_KB - 1) / CT_KB);
-  if ((long long)P + t.bm >= (1ll << 31) || (long long)K + CT_KB >= (1ll << 31)) return f;
-  // A launch of this kernel costs about 30 us more than one of the table kernels before it is at full rate
-  // (tables, tensor memory, tiles of 128 x 256): below 4e8 products, or with less than half of a tile's
-  // rows or columns used, it does not win that back.
-  if (sw().codes < 0 && ((double)P * Q * K * batch < 4e8 || P < 96 || Q < 48)) return f;
-  f.grid = (int)std::min<long long>(sms, std::max<long long>(1, f.iters / 2));
-  f.slot_bytes = (size_t)f.grid * 2 * t.slot_bytes;
-  f.counter_bytes = ((size_t)f.tiles * sizeof(int) + 255) / 256 * 256;
+  if ((long long)P + tile.bm >= (1ll << 31) || (long long)K + CT_KB >= (1ll << 31) || f.iters >= (1ll << 31) - 1) return f;
+  // Runs of at least two blocks; and no more runs per tile than pay for themselves: a run more shortens the others by
+  // iters / grid^2 blocks and costs the tile's last one 1 / tiles of a parked tile.
+  const double best = std::sqrt((double)f.iters * (double)f.tiles * kCodeBlockUs[f.shape] / kCodeShareUs[f.shape]);
+  f.grid = (int)std::min<double>((double)std::min<long long>(sms / 2, std::max<long long>(1, f.iters / 2)), std::max(1.0, best));
+  if (f.grid < 1) return f;
+  // Below 1e8 products both paths take a few tens of microseconds, and the estimates do not tell them apart.
+  // Batched products stay on the table kernels: attention cuts softmax weights down to the table's few mantissa bits for
+  // its next product, so a last-bit change of the scores shows as 2e-3 of the result's root mean square there; and a
+  // tile's 256 rows are of one product (512 of 128 x 128 x 64: MIT_7 65 / 137 us, MBM_7 109 / 88 us).
+  const double products = (double)P * Q * K * batch;
+  if (w.codes < 0 && (batch > 1 || products < 1e8 || code_us(f, t) > 0.95 * table_us(products, K, t))) return f;
+  f.slot_bytes = (size_t)f.grid * 2 * tile.slot_bytes;
+  f.counter_bytes = ((size_t)f.tiles * 2 * sizeof(int) + 255) / 256 * 256;
   f.use = 1;
   return f;
 }
@@ -740,10 +772,11 @@ int launch_codes(cudaStream_t st, const Params& p, const CodePlan& f, bool fgrad
   return AMSIM_OK;
 }
 
-// 128-slot tables (all 7 bits of a mantissa matter, MIT_7) cost twice the codes per product: no faster than
-// the additive-table kernels, which need no lookups.
 bool codes_eligible(const Params& p, bool exact) {
-  return !exact && p.ct_slots > 0 && (p.ct_slots <= 64 || sw().codes > 0) && (p.lut_mode == LM_SMEM || p.lut_mode == LM_ADD);
+  return !exact && p.ct_slots > 0 && (p.lut_mode == LM_SMEM || p.lut_mode == LM_ADD);
+}
+CodeTraits code_traits(const Params& p, bool fgrad) {
+  return {p.ct_slots, p.lut_mode == LM_ADD, fgrad, !p.v_trans && p.g.SC % 4 != 0};
 }
 
 int launch_gather(cudaStream_t st, Params& p, int batch, bool exact, int device) {
@@ -751,7 +784,7 @@ int launch_gather(cudaStream_t st, Params& p, int batch, bool exact, int device)
   fill_bounds(p, device, nullptr, 0);
   if ((long long)p.P >= (1ll << 31) - 256) return fail(AMSIM_ERR_UNSUPPORTED, "more than 2^31 output rows");
   if (codes_eligible(p, exact)) {
-    const CodePlan f = plan_codes(p.P, p.Q, p.K, batch, sm_count(device));
+    const CodePlan f = plan_codes(p.P, p.Q, p.K, batch, sm_count(device), code_traits(p, false));
     if (f.use) {
       cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
       CUDA_TRY(cudaStreamIsCapturing(st, &cap));
@@ -761,7 +794,7 @@ int launch_gather(cudaStream_t st, Params& p, int batch, bool exact, int device)
       if (rc) return rc;
       if (sc.ws) {
         char* base = reinterpret_cast<char*>(sc.ws);
-        const bool clean = !sc.pooled && (size_t)f.tiles <= kPersistentCounters;
+        const bool clean = !sc.pooled && (size_t)f.tiles * 2 <= kPersistentCounters;
         char* counters = clean ? base : base + kPersistentCounterBytes + f.slot_bytes;
         Params q = p;
         fill_bounds(q, device, base, bytes);
@@ -897,7 +930,7 @@ size_t fgrad_workspace(int P, int Q, int K, bool exact, int sms) {
         if (np) need = std::max(need, plan_fgrad(P, Q, K, false, np, sms).ws_bytes);
       }
     }
-    const CodePlan c = plan_codes(P, Q, K, 1, sms);
+    const CodePlan c = plan_codes(P, Q, K, 1, sms, kCodeTraitsAny);
     if (c.use) need = std::max(need, c.counter_bytes + c.slot_bytes);
   }
   return need;
@@ -995,7 +1028,7 @@ int launch_fgrad(cudaStream_t st, Params& p, bool exact, void* ws, size_t ws_byt
   const int sms = sm_count(device);
   if (codes_eligible(p, exact)) {
     // (a caller whose workspace does not hold the parked tiles takes the split-K kernels below)
-    const CodePlan c = plan_codes(p.P, p.Q, p.K, 1, sms);
+    const CodePlan c = plan_codes(p.P, p.Q, p.K, 1, sms, code_traits(p, true));
     if (c.use && ws && aligned16(ws) && ws_bytes >= c.counter_bytes + c.slot_bytes) {
       Params q = p;
       fill_bounds(q, device, ws, c.counter_bytes + c.slot_bytes);

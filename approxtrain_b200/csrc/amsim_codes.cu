@@ -11,37 +11,37 @@
 namespace amsim {
 namespace {
 
-template <int S, int MT, int BN>
+template <int S, int BN>
 cudaError_t code_launch_t(cudaStream_t st, const CodeParams& cp, int device) {
-  using L = CodeSmem<S, MT, BN>;
+  using L = CodeSmem<S, BN>;
   static std::mutex mu;
   static size_t allowed[64] = {};
   const size_t smem = L::bytes(cp.rows_v, cp.rows_u);
   if (device >= 0 && device < 64) {
     std::lock_guard<std::mutex> lk(mu);
     if (allowed[device] < smem) {
-      const cudaError_t e = cudaFuncSetAttribute(code_gemm<S, MT, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      const cudaError_t e = cudaFuncSetAttribute(code_gemm<S, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
       allowed[device] = smem;
     }
   }
-  code_gemm<S, MT, BN><<<cp.prm.sk_grid, L::NT, smem, st>>>(cp);
+  code_gemm<S, BN><<<2 * cp.prm.sk_grid, L::NT, smem, st>>>(cp);
   return cudaGetLastError();
 }
 
 template <int S>
 cudaError_t code_launch_s(cudaStream_t st, const CodeParams& cp, int shape, int device) {
-  if (shape == 0) return code_launch_t<S, 1, 256>(st, cp, device);
-  if (shape == 1) return code_launch_t<S, 2, 128>(st, cp, device);
-  return code_launch_t<S, 2, 64>(st, cp, device);
+  if (shape == 0) return code_launch_t<S, 256>(st, cp, device);
+  if (shape == 1) return code_launch_t<S, 128>(st, cp, device);
+  return code_launch_t<S, 64>(st, cp, device);
 }
 
 }  // namespace
 
 CodeTile code_tile(int shape) {
-  if (shape == 0) return {128, 256, (size_t)CodeAcc<64, 1, 256>::SLOT_FLOATS * 4};
-  if (shape == 1) return {256, 128, (size_t)CodeAcc<64, 2, 128>::SLOT_FLOATS * 4};
-  return {256, 64, (size_t)CodeAcc<64, 2, 64>::SLOT_FLOATS * 4};
+  if (shape == 0) return {CT_ROWS, 256, (size_t)CodeAcc<64, 256>::SLOT_FLOATS * 8};
+  if (shape == 1) return {CT_ROWS, 128, (size_t)CodeAcc<64, 128>::SLOT_FLOATS * 8};
+  return {CT_ROWS, 64, (size_t)CodeAcc<64, 64>::SLOT_FLOATS * 8};
 }
 
 cudaError_t code_gemm_launch(cudaStream_t st, const CodeParams& cp, int shape, int device) {

@@ -20,31 +20,37 @@
 // reference-order result the path is within 4e-8 (short reductions) to 3e-7 (10^5 steps), like the
 // split sums of the shared-memory kernels.
 //
-// Rates: 64 code steps of a 128 x 256 tile take 128 clocks (measured, also with all multiprocessors
-// busy), so 64-slot tables run at most 256 products per clock and multiprocessor, 8 times the 32
-// table lookups per clock that bound the shared-memory kernels.  What bounds this kernel is making
-// the operands: per reduction step and operand row S / 2 bytes of codes are looked up in a table,
-// sign-flipped and stored, all through the 128-byte/clock path to shared memory that the tensor
-// core reads from too (266 wavefronts per step of a 128 x 256 tile, 64-slot table).  Hence the codes
-// of V go to tensor memory instead (the product takes its first operand from there).
+// Two CTAs (one pair of multiprocessors) share a tile of 256 rows and up to 256 columns (tcgen05 cta_group::2): each
+// encodes 128 rows of V and half the columns of U, the tensor cores read both halves, and the CTA of rank 0 issues.
+// Every CTA needs the scale bytes of all columns; the other half's arrive by st.async on its own barrier.
 //
-// One CTA per multiprocessor: 12 warps own 32 operand rows each (4 MT warps the rows of V, the rest
-// the columns of U): a warp fetches the raw FP32 elements of its rows with its own cp.async double
-// buffer, encodes them, and signals the stage; one more warp issues the matrix products.  No barrier
-// spans the CTA inside the loop.  Work is dealt out in equal runs of (tile, 16-step block) pairs as
-// in gather_gemm's balanced mode.
+// Rates: 64 code steps of a 256 x 256 tile take a pair 128 clocks, so 64-slot tables run at most 256 products per clock
+// and multiprocessor, 8 times the 32 table lookups per clock that bound the shared-memory kernels.  What bounds this
+// kernel is making the operands: per reduction step and operand row S / 2 bytes of codes are looked up in a table,
+// sign-flipped and stored.  The codes of V go to tensor memory (the product takes its first operand from there), the
+// codes of U to shared memory.  With one CTA per tile of 128 x 256 every multiprocessor encoded 384 rows a step, with
+// pairs 256.  The tensor pipe is active a third of the time; the operand warps' chains of lookups, stores and barrier
+// operations are the rest.
 //
-// Measured (MBM_7, B200): 3x3 256 -> 256 on 64 x 14 x 14, forward 1255 -> 318 us, filter gradient
-// 1250 -> 349 us (gather_gemm / wide_fgrad -> code_gemm).
+// 32 rows or columns belong to two warps, which make the stages of a 16-step block's halves: a warp fetches the raw FP32
+// elements of its rows with its own cp.async double buffer, encodes them, and signals the stage; one more warp issues
+// the matrix products (rank 0) or forwards the signals (rank 1).  No barrier spans the CTA inside the loop.  Work is
+// dealt out in equal runs of (tile, 16-step block) pairs as in gather_gemm's balanced mode.
+//
+// Measured (B200, table kernels / one CTA per tile / pairs): 3x3 256 -> 256 on 64 x 14 x 14 with MBM_7, forward
+// 1255 / 318 / 272 us, filter gradient 1250 / 349 / 283 us; 8192 x 512 x 2048 with MIT_7 929 / - / 581 us.
 #pragma once
 #include "amsim_kernels.cuh"
 #include "amsim_wide.cuh"
 
 namespace amsim {
 
-constexpr int CT_KB = 16;        // reduction steps per block (one cp.async buffer of a warp)
+constexpr int CT_KB = 16;        // reduction steps per block; a warp fetches and encodes one half of each
+constexpr int CT_HALF = CT_KB / 2;
+constexpr int CT_RAW = 32 * CT_HALF * 4;  // one cp.async buffer of a warp
+constexpr int CT_ROWS = 256;     // rows of a CTA pair's tile
 constexpr int CT_CHUNK = 8;      // blocks summed in tensor memory before they go to the FP32 partial tile
-constexpr int CT_MAXSPIN = 1 << 22;  // bound on every wait (a wait gives up, the kernel drains and reports)
+constexpr int CT_MAXSPIN = 1 << 20;  // bound on every wait (a wait gives up, the kernel drains and reports)
 
 // How an operand's elements sit in memory.
 constexpr int CT_KVEC = 0;   // 16-byte groups of four consecutive reduction steps of one row
@@ -74,27 +80,25 @@ struct CodeCfg {
   static constexpr int STAGES_PER_KB = CT_KB / KS;
 };
 
-template <int S, int MT, int BN>
+template <int S, int BN>
 struct CodeSmem {
   using C = CodeCfg<S>;
-  static constexpr int BM = 128 * MT;
-  static constexpr int NW = 4 * MT + BN / 32;
+  static constexpr int GU = BN / 64;              // 32-column groups of U per CTA (half of the pair's columns)
+  static constexpr int NW = 2 * (4 + GU);         // two warps per group of 32 rows or columns
   static constexpr int NT = 32 * (NW + 1);
-  static constexpr int NBH = (BN + 127) / 128;    // 512-byte scale chunks of U per word
-  // stages in flight: a stage lives from the encoding of its rows to the end of its products (about
-  // 2000 clocks, of which the products take 512), so two stages leave the tensor core waiting
-  static constexpr int NST = MT == 2 && BN == 128 ? 3 : S == 128 ? 3 : 4;
-  static constexpr int CODE_BYTES = BN * 128;     // the codes of V go to tensor memory
-  static constexpr int SF_BYTES = (MT + NBH) * C::W * 512;
+  static constexpr int NBH = (BN + 127) / 128;    // 512-byte scale chunks of U per word (both halves: every CTA needs all)
+  static constexpr int NST = BN == 256 ? 6 : 8;   // stages in flight: tensor memory and shared memory hold no more
+  static constexpr int CODE_BYTES = BN / 2 * 128; // the codes of V go to tensor memory
+  static constexpr int SF_BYTES = (1 + NBH) * C::W * 512;
   static constexpr int OFF_SF = NST * CODE_BYTES;
   static constexpr int OFF_RAW = OFF_SF + NST * SF_BYTES;
   // tensor memory columns: accumulators, NST stages of V codes, two sets of scales
-  static constexpr int T_CODES = MT * BN;
-  static constexpr int T_SF = T_CODES + NST * MT * 32;
-  static constexpr int SF_COLS = (MT + NBH) * C::W * 4;
+  static constexpr int T_CODES = BN;
+  static constexpr int T_SF = T_CODES + NST * 32;
+  static constexpr int SF_COLS = (1 + NBH) * C::W * 4;
   static_assert(T_SF + 2 * SF_COLS <= 512, "tensor memory");
-  static constexpr int OFF_ROW = OFF_RAW + NW * 2 * 2048;
-  static constexpr int OFF_TAB = OFF_ROW + BM * 16;
+  static constexpr int OFF_ROW = OFF_RAW + NW * 2 * CT_RAW;
+  static constexpr int OFF_TAB = OFF_ROW + 8 * 512;
   static size_t bytes(int rows_v, int rows_u) {
     return 1024 + OFF_TAB + (size_t)(rows_v + 1 + rows_u + 1) * C::CH * C::REP * 16;
   }
@@ -104,12 +108,38 @@ struct CodeSmem {
 __device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
+// Address in the cluster's shared memory of this CTA's `addr` in the CTA of that rank.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// bar: an address in the cluster's shared memory
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Stores a word in the other CTA's shared memory and counts its four bytes there (both addresses the cluster's).
+__device__ __forceinline__ void st_async_remote(uint32_t addr, uint32_t v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {  // (does not wait)
+  uint32_t ok;
+  asm volatile("{.reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
@@ -119,35 +149,56 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46) |
          ((uint64_t)layout << 61);
 }
-// kind::mxf4: E2M1 codes, E8M0 scales, FP32 accumulator; M = 128
+// kind::mxf4: E2M1 codes, E8M0 scales, FP32 accumulator; M = 256 over the two CTAs
 __host__ __device__ constexpr uint32_t code_idesc(int n) {
-  return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | (1u << 27);
+  return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | (1u << 28);
 }
 __device__ __forceinline__ void mma_codes(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb,
                                           uint32_t accumulate) {
   asm volatile(
       "{.reg .pred p; setp.ne.b32 p, %6, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], %2, %3, [%4], [%5], p;}" ::"r"(d),
+      "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], %2, %3, [%4], [%5], p;}" ::"r"(d),
       "r"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void scales_to_tmem(uint32_t taddr, uint64_t desc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
 }
+// Arrives at this barrier of both CTAs when the products issued so far are done.
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"((uint16_t)3) : "memory");
 }
-__device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_load16(uint32_t taddr, float (&v)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+        "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+      : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ bool elect_lane() {
   uint32_t e;
   asm volatile("{.reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p;}" : "=r"(e));
   return e != 0;
+}
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+// (the clobbers keep reads of what other lanes have copied in behind the wait and the warp barrier)
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
 }
 __device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
@@ -194,15 +245,16 @@ __device__ __forceinline__ void copy_code_table(uint4* dst, const uint4* __restr
   }
 }
 
-// Fetches the 32 rows x 16 reduction steps a warp encodes, raw FP32, into its 2 KB buffer:
-// CT_K*: row r at 64 r, its four 16-byte groups at (group ^ (r >> 1 & 3)); CT_R*: step k at 128 k.
+// Fetches the 32 rows x 8 reduction steps (one half of a block) a warp encodes, raw FP32, into its 1 KB buffer:
+// CT_K*: row r at 32 r, its two 16-byte groups at (group ^ (r >> 2 & 1)); CT_R*: step k at 128 k.
 struct RowFetch {
+  int k_at;              // first step of this warp's half within a block
   int e_kh, e_kw, e_ch;  // filter tap of this lane's row (group) of a filter gradient
   bool e_ok;
-  // Stepping (cp.step): where a block of 16 steps never straddles a filter tap, the four 16-byte groups a
+  // Stepping (cp.step): where a block of 16 steps never straddles a filter tap, the two 16-byte groups a
   // lane copies per block sit at offsets that advance by a constant until the tap ends.  (Decoding the tap and
   // the rows anew for every block took as many instructions as encoding a stage.)
-  int off[4];            // element offsets of the next block's groups
+  int off[2];            // element offsets of the next block's groups
   int left;              // blocks left in the tap
   uint32_t okm;          // bit i: group i exists
 
@@ -237,10 +289,10 @@ struct RowFetch {
     __syncwarp();
   }
 
-  __device__ __forceinline__ void issue4(const Params& prm, int which, const float* __restrict__ base, int step, uint32_t dst,
+  __device__ __forceinline__ void issue(const Params& prm, int which, const float* __restrict__ base, int step, uint32_t dst,
                                          uint32_t dst_step) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 2; ++i) {
       bool ok = (okm >> i) & 1u;
       const float* src = base + (ok ? off[i] : 0);
       ok = ok && AMSIM_IN(prm, which, src, float4);
@@ -249,55 +301,55 @@ struct RowFetch {
     }
     --left;
   }
-  // CT_KVEC patch rows: group i of a lane = row 8 i + lane / 4, steps 4 (lane % 4)...
+  // CT_KVEC patch rows: group i of a lane = row 16 i + lane / 2, steps 4 (lane % 2)...
   __device__ __forceinline__ void step_v(const CodeParams& cp, const float* __restrict__ Vg, int kb, const int4* rowinfo,
                                          uint32_t dst, int lane) {
     const Params& prm = cp.prm;
     const Gather& g = prm.g;
     if (left == 0) {
-      const int k = kb * CT_KB;
+      const int k = kb * CT_KB + k_at;
       const int tap = (int)fdiv((uint32_t)k, g.d_sc), ch = k - tap * g.SC;
       const int kh = (int)fdiv((uint32_t)tap, g.d_kw), kw = tap - kh * g.KW;
-      left = (g.SC - ch) / CT_KB;
+      left = (g.SC - ch + k_at) / CT_KB;
       okm = 0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int4 ri = rowinfo[i * 8 + (lane >> 2)];
+      for (int i = 0; i < 2; ++i) {
+        const int4 ri = rowinfo[i * 16 + (lane >> 1)];
         const int u = ri.x + kh, v = ri.y + kw;
         if ((unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w) okm |= 1u << i;
-        off[i] = ri.z + (u * g.SW + v) * g.SC + ch + 4 * (lane & 3);
+        off[i] = ri.z + (u * g.SW + v) * g.SC + ch + 4 * (lane & 1);
       }
     }
-    const int r = lane >> 2;
-    issue4(prm, BUF_V, Vg, CT_KB, dst + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4), 8 * 64);
+    const int r = lane >> 1;
+    issue(prm, BUF_V, Vg, CT_KB, dst + r * 32 + (((lane & 1) ^ ((r >> 2) & 1)) << 4), 16 * 32);
   }
-  // CT_RVEC: group i = step 4 i + lane / 8, rows 4 (lane % 8)...; CT_KVEC: as above
+  // CT_RVEC: group i of a lane = step 4 i + lane / 8, rows 4 (lane % 8)...; CT_KVEC: as above
   __device__ __forceinline__ void step_u(const CodeParams& cp, const float* __restrict__ Ug, int first, int kb, uint32_t dst,
                                          int lane) {
     const Params& prm = cp.prm;
     const bool rvec = cp.u_mode == CT_RVEC;
     if (left == 0) {
-      const int k = kb * CT_KB;
+      const int k = kb * CT_KB + k_at;
       if (cp.fgrad) {
         left = INT32_MAX;
       } else {
         const int tap = (int)fdiv((uint32_t)k, prm.g.d_sc);
-        left = (prm.g.SC - (k - tap * prm.g.SC)) / CT_KB;
+        left = (prm.g.SC - (k - tap * prm.g.SC) + k_at) / CT_KB;
       }
       const int base = (int)u_offset(cp, k);
       okm = 0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int q = first + (rvec ? 4 * (lane & 7) : i * 8 + (lane >> 2));
+      for (int i = 0; i < 2; ++i) {
+        const int q = first + (rvec ? 4 * (lane & 7) : i * 16 + (lane >> 1));
         if (q < prm.Q) okm |= 1u << i;
-        off[i] = base + (rvec ? (4 * i + (lane >> 3)) * prm.u_sk + q : q * prm.u_sq + 4 * (lane & 3));
+        off[i] = base + (rvec ? (4 * i + (lane >> 3)) * prm.u_sk + q : q * prm.u_sq + 4 * (lane & 1));
       }
     }
     if (rvec) {
-      issue4(prm, BUF_U, Ug, CT_KB * prm.u_sk, dst + lane * 16, 512);
+      issue(prm, BUF_U, Ug, CT_KB * prm.u_sk, dst + lane * 16, 512);
     } else {
-      const int r = lane >> 2;
-      issue4(prm, BUF_U, Ug, CT_KB, dst + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4), 8 * 64);
+      const int r = lane >> 1;
+      issue(prm, BUF_U, Ug, CT_KB, dst + r * 32 + (((lane & 1) ^ ((r >> 2) & 1)) << 4), 16 * 32);
     }
   }
 
@@ -308,8 +360,8 @@ struct RowFetch {
     if (cp.fgrad) {
       if (cp.v_mode == CT_RVEC) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int kl = i * 4 + (lane >> 3), pix = kb * CT_KB + kl;
+        for (int i = 0; i < 2; ++i) {
+          const int kl = i * 4 + (lane >> 3), pix = kb * CT_KB + k_at + kl;
           const uint32_t n = fdiv((uint32_t)pix, g.d_img);
           const uint32_t rem = (uint32_t)pix - n * (uint32_t)(g.PH * g.PW);
           const uint32_t a = fdiv(rem, g.d_pw);
@@ -322,8 +374,8 @@ struct RowFetch {
         }
       } else {
 #pragma unroll 4
-        for (int kl = 0; kl < CT_KB; ++kl) {
-          const int pix = kb * CT_KB + kl;
+        for (int kl = 0; kl < CT_HALF; ++kl) {
+          const int pix = kb * CT_KB + k_at + kl;
           const uint32_t n = fdiv((uint32_t)pix, g.d_img);
           const uint32_t rem = (uint32_t)pix - n * (uint32_t)(g.PH * g.PW);
           const uint32_t a = fdiv(rem, g.d_pw);
@@ -340,8 +392,8 @@ struct RowFetch {
     if (prm.v_trans) {  // V[p, k] at V[k * v_ld + p]
       if (cp.v_mode == CT_RVEC) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int kl = i * 4 + (lane >> 3), k = kb * CT_KB + kl, p = first + 4 * (lane & 7);
+        for (int i = 0; i < 2; ++i) {
+          const int kl = i * 4 + (lane >> 3), k = kb * CT_KB + k_at + kl, p = first + 4 * (lane & 7);
           bool ok = k < prm.K && p < prm.P;
           const float* src = ok ? Vg + (long long)k * prm.v_ld + p : Vg;
           ok = ok && AMSIM_IN(prm, BUF_V, src, float4);
@@ -349,8 +401,8 @@ struct RowFetch {
         }
       } else {
 #pragma unroll 4
-        for (int kl = 0; kl < CT_KB; ++kl) {
-          const int k = kb * CT_KB + kl, p = first + lane;
+        for (int kl = 0; kl < CT_HALF; ++kl) {
+          const int k = kb * CT_KB + k_at + kl, p = first + lane;
           bool ok = k < prm.K && p < prm.P;
           const float* src = ok ? Vg + (long long)k * prm.v_ld + p : Vg;
           ok = ok && AMSIM_IN(prm, BUF_V, src, float);
@@ -360,7 +412,7 @@ struct RowFetch {
       return;
     }
     const bool vec = cp.v_mode == CT_KVEC;
-    const int kl = vec ? 4 * (lane & 3) : (lane & 15), k = kb * CT_KB + kl;
+    const int kl = vec ? 4 * (lane & 1) : (lane & 7), k = kb * CT_KB + k_at + kl;
     const uint32_t tap = fdiv((uint32_t)k, g.d_sc);
     const int ch = k - (int)tap * g.SC;
     const int kh = (int)fdiv(tap, g.d_kw);
@@ -368,27 +420,27 @@ struct RowFetch {
     const bool k_ok = k < prm.K;
     if (vec) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = i * 8 + (lane >> 2);
+      for (int i = 0; i < 2; ++i) {
+        const int r = i * 16 + (lane >> 1);
         const int4 ri = rowinfo[r];
         const int u = ri.x + kh, v = ri.y + kw;
         bool ok = k_ok && (unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w;
         const long long nb = ((long long)ri.w << 32) | (uint32_t)ri.z;
         const float* src = ok ? Vg + nb + ((long long)(u * g.SW + v) * g.SC + ch) : Vg;
         ok = ok && AMSIM_IN(prm, BUF_V, src, float4);
-        cp_async16n(dst + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4), src, ok ? 16 : 0);
+        cp_async16n(dst + r * 32 + (((lane & 1) ^ ((r >> 2) & 1)) << 4), src, ok ? 16 : 0);
       }
     } else {
 #pragma unroll 4
-      for (int i = 0; i < 16; ++i) {
-        const int r = i * 2 + (lane >> 4);
+      for (int i = 0; i < 8; ++i) {
+        const int r = i * 4 + (lane >> 3);
         const int4 ri = rowinfo[r];
         const int u = ri.x + kh, v = ri.y + kw;
         bool ok = k_ok && (unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w;
         const long long nb = ((long long)ri.w << 32) | (uint32_t)ri.z;
         const float* src = ok ? Vg + nb + ((long long)(u * g.SW + v) * g.SC + ch) : Vg;
         ok = ok && AMSIM_IN(prm, BUF_V, src, float);
-        cp_async4(dst + r * 64 + (((kl >> 2) ^ ((r >> 1) & 3)) << 4) + (kl & 3) * 4, src, ok);
+        cp_async4(dst + r * 32 + (((kl >> 2) ^ ((r >> 2) & 1)) << 4) + (kl & 3) * 4, src, ok);
       }
     }
   }
@@ -410,39 +462,39 @@ struct RowFetch {
     const Params& prm = cp.prm;
     if (cp.u_mode == CT_RVEC) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int kl = i * 4 + (lane >> 3), k = kb * CT_KB + kl, q = first + 4 * (lane & 7);
+      for (int i = 0; i < 2; ++i) {
+        const int kl = i * 4 + (lane >> 3), k = kb * CT_KB + k_at + kl, q = first + 4 * (lane & 7);
         bool ok = k < prm.K && q < prm.Q;
         const float* src = ok ? Ug + u_offset(cp, k) + q : Ug;
         ok = ok && AMSIM_IN(prm, BUF_U, src, float4);
         cp_async16n(dst + kl * 128 + (lane & 7) * 16, src, ok ? 16 : 0);
       }
     } else if (cp.u_mode == CT_KVEC) {
-      const int k = kb * CT_KB + 4 * (lane & 3);
+      const int k = kb * CT_KB + k_at + 4 * (lane & 1);
       const float* col = Ug + u_offset(cp, k);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = i * 8 + (lane >> 2), q = first + r;
+      for (int i = 0; i < 2; ++i) {
+        const int r = i * 16 + (lane >> 1), q = first + r;
         bool ok = k < prm.K && q < prm.Q;
         const float* src = ok ? col + (long long)q * prm.u_sq : Ug;
         ok = ok && AMSIM_IN(prm, BUF_U, src, float4);
-        cp_async16n(dst + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4), src, ok ? 16 : 0);
+        cp_async16n(dst + r * 32 + (((lane & 1) ^ ((r >> 2) & 1)) << 4), src, ok ? 16 : 0);
       }
     } else if (cp.u_mode == CT_KSCL) {
-      const int kl = lane & 15, k = kb * CT_KB + kl;
+      const int kl = lane & 7, k = kb * CT_KB + k_at + kl;
       const float* col = Ug + u_offset(cp, k);
 #pragma unroll 4
-      for (int i = 0; i < 16; ++i) {
-        const int r = i * 2 + (lane >> 4), q = first + r;
+      for (int i = 0; i < 8; ++i) {
+        const int r = i * 4 + (lane >> 3), q = first + r;
         bool ok = k < prm.K && q < prm.Q;
         const float* src = ok ? col + (long long)q * prm.u_sq : Ug;
         ok = ok && AMSIM_IN(prm, BUF_U, src, float);
-        cp_async4(dst + r * 64 + (((kl >> 2) ^ ((r >> 1) & 3)) << 4) + (kl & 3) * 4, src, ok);
+        cp_async4(dst + r * 32 + (((kl >> 2) ^ ((r >> 2) & 1)) << 4) + (kl & 3) * 4, src, ok);
       }
     } else {
 #pragma unroll 4
-      for (int kl = 0; kl < CT_KB; ++kl) {
-        const int k = kb * CT_KB + kl, q = first + lane;
+      for (int kl = 0; kl < CT_HALF; ++kl) {
+        const int k = kb * CT_KB + k_at + kl, q = first + lane;
         bool ok = k < prm.K && q < prm.Q;
         const float* src = ok ? Ug + u_offset(cp, k) + (long long)q * prm.u_sq : Ug;
         ok = ok && AMSIM_IN(prm, BUF_U, src, float);
@@ -473,25 +525,25 @@ __device__ __forceinline__ void store_out4(const Params& prm, float* __restrict_
 }
 
 // Share of a thread in draining and writing a tile: 16-column units u = g, g + NG, ... of the tile (g = warp / 4), of
-// the tile row 32 * (warp % 4) + lane of 128-row subtile u / (BN / 16).
-template <int S, int MT, int BN>
+// the CTA's tile row 32 * (warp % 4) + lane.
+template <int S, int BN>
 struct CodeAcc {
-  static constexpr int NG = CodeSmem<S, MT, BN>::NW / 4;
-  static constexpr int UNITS = MT * BN / 16;
+  static constexpr int NG = CodeSmem<S, BN>::NW / 4;
+  static constexpr int UNITS = BN / 16;
   static constexpr int UPT = (UNITS + NG - 1) / NG;
   static constexpr int NTE = NG * 128;                 // threads that drain
-  static constexpr int SLOT_FLOATS = UPT * 16 * NTE;   // one parked tile
+  static constexpr int SLOT_FLOATS = UPT * 16 * NTE;   // one parked tile of a CTA
 };
 
-template <int S, int MT, int BN>
-__global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __grid_constant__ CodeParams cp) {
+template <int S, int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT, 1) code_gemm(const __grid_constant__ CodeParams cp) {
   using C = CodeCfg<S>;
-  using L = CodeSmem<S, MT, BN>;
-  using A = CodeAcc<S, MT, BN>;
-  constexpr int NW = L::NW, BM = L::BM, KS = C::KS, W = C::W, CH = C::CH, REP = C::REP, NST = L::NST;
+  using L = CodeSmem<S, BN>;
+  using A = CodeAcc<S, BN>;
+  constexpr int NW = L::NW, GU = L::GU, KS = C::KS, W = C::W, CH = C::CH, REP = C::REP, NST = L::NST;
   constexpr int NG = A::NG, UPT = A::UPT;
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  __shared__ uint64_t bars[2 * NST + 2];
+  __shared__ uint64_t bars[3 * NST + 2];
   __shared__ uint32_t tmem_holder;
   __shared__ int flag_s;
   const Params& prm = cp.prm;
@@ -500,21 +552,25 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
   uint8_t* const smem = smem_raw + (smem0 - smem_addr(smem_raw));
   const int t = threadIdx.x, lane = t & 31;
   const int w = __shfl_sync(0xffffffffu, t >> 5, 0);
+  const uint32_t rank = blockIdx.x & 1u;  // in the pair; the CTA of rank 0 issues the products of both
+  const int pair = blockIdx.x >> 1;
   const uint32_t bar0 = smem_addr(bars);
-  const uint32_t bar_full = bar0, bar_empty = bar0 + 8 * NST, bar_done = bar0 + 16 * NST, bar_free = bar_done + 8;
+  const uint32_t bar_full = bar0, bar_empty = bar0 + 8 * NST, bar_peer = bar0 + 16 * NST, bar_done = bar0 + 24 * NST,
+                 bar_free = bar_done + 8;
 
   if (t == 0) {
     for (int i = 0; i < NST; ++i) {
-      mbar_init(bar_full + 8 * i, NW);
+      mbar_init(bar_full + 8 * i, NW / 2);  // half of the warps make a stage; the other CTA adds its scale bytes
+      mbar_init(bar_peer + 8 * i, 1);       // (rank 0) the other CTA's stage is full
       mbar_init(bar_empty + 8 * i, 1);
     }
     mbar_init(bar_done, 1);
-    mbar_init(bar_free, 4 * NG);
+    mbar_init(bar_free, 2 * 4 * NG);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (w == NW) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_holder)) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_holder)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   uint4* const tab_v = reinterpret_cast<uint4*>(smem + L::OFF_TAB);
   uint4* const tab_u = tab_v + (cp.rows_v + 1) * CH * REP;
@@ -522,24 +578,44 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
   copy_code_table<CH, REP>(tab_u, cp.tab_u, cp.rows_u + 1, t, L::NT);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_barrier();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_holder, 0);
 
   const int nkb_all = (prm.K + CT_KB - 1) / CT_KB;
-  long long run_at = balanced_begin(blockIdx.x, prm.sk_iters, prm.sk_grid);
-  const long long run_end = balanced_begin((long long)blockIdx.x + 1, prm.sk_iters, prm.sk_grid);
-  auto decode_tile = [&](long long at, int& tp, int& tq, int& tz, int& kb0, int& kb1) {
-    const long long tile = at / nkb_all;
-    kb0 = (int)(at - tile * nkb_all);
-    kb1 = kb0 + (int)min((long long)(nkb_all - kb0), run_end - at);
-    tq = (int)(tile % prm.sk_qtiles);
-    const long long rest = tile / prm.sk_qtiles;
-    tp = (int)(rest % prm.sk_ptiles);
-    tz = (int)(rest / prm.sk_ptiles);
+  int run_at = (int)balanced_begin(pair, prm.sk_iters, prm.sk_grid);  // (the launch has fewer than 2^31 blocks)
+  const int run_end = (int)balanced_begin((long long)pair + 1, prm.sk_iters, prm.sk_grid);
+  auto decode_tile = [&](int at, int& tp, int& tq, int& tz, int& kb0, int& kb1) {
+    const uint32_t tile = (uint32_t)at / (uint32_t)nkb_all;
+    kb0 = at - (int)tile * nkb_all;
+    kb1 = kb0 + min(nkb_all - kb0, run_end - at);
+    const uint32_t rest = tile / (uint32_t)prm.sk_qtiles;
+    tq = (int)(tile - rest * (uint32_t)prm.sk_qtiles);
+    tz = (int)(rest / (uint32_t)prm.sk_ptiles);
+    tp = (int)rest - tz * prm.sk_ptiles;
   };
+  // columns of U in the products of tile column tq; each CTA encodes one half of them
+  auto tile_columns = [&](int tq) { return min(BN, (prm.Q - tq * BN + 63) / 64 * 64); };
   Waiter wt{cp.stuck, false};
 
-  if (w == NW) {
+  if (w == NW && rank != 0) {
+    // ---- forwards "stage full" of this CTA to the issuing one: one warp fences for all, and the operand warps signal
+    // inside their CTA only (a proxy fence and a cluster-wide release in every one of them, with its own stores in
+    // flight, made 3x3 256 -> 256 on 64 x 14 x 14 take 483 us instead of 316)
+    const uint32_t lead = cluster_addr(bar_peer, 0);
+    uint32_t b = 0, phase = 0;
+    const long long stages = (long long)(run_end - run_at) * C::STAGES_PER_KB;
+    for (long long i = 0; i < stages; ++i) {
+      wt.wait_warp(bar_full + 8 * b, phase);
+      asm volatile("tcgen05.fence::after_thread_sync;\nfence.proxy.async.shared::cta;\ntcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_remote(lead + 8 * b);
+      if (++b == NST) {
+        b = 0;
+        phase ^= 1;
+      }
+    }
+  } else if (w == NW) {
     // ---- issue warp: moves the scales to tensor memory and issues the products --------------------
     // The whole warp walks the loop on warp-uniform values and one elected lane issues, so descriptors
     // and addresses stay in uniform registers (with a single-lane loop the moves into uniform registers
@@ -551,37 +627,32 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
       int tp, tq, tz, kb0, kb1;
       decode_tile(run_at, tp, tq, tz, kb0, kb1);
       run_at += kb1 - kb0;
-      const int n = min(BN, (prm.Q - tq * BN + 31) / 32 * 32);
-      const int mts = min(MT, (prm.P - tp * BM + 127) / 128);
-      const uint32_t idesc = code_idesc(n);
+      const uint32_t idesc = code_idesc(tile_columns(tq));
       for (int kb = kb0; kb < kb1; kb += CT_CHUNK, ++chunk) {
         const int stages = (min(kb1, kb + CT_CHUNK) - kb) * C::STAGES_PER_KB;
         wt.wait_warp(bar_free, (chunk & 1) ^ 1);
         uint32_t accumulate = 0;
 #pragma unroll 1
         for (int i = 0; i < stages; ++i) {
-          wt.wait_warp(bar_full + 8 * b, phase);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          wt.wait(bar_full + 8 * b, phase);
+          wt.wait_warp(bar_peer + 8 * b, phase);
+          asm volatile("tcgen05.fence::after_thread_sync;\nfence.proxy.async.shared::cta;" ::: "memory");
           const uint64_t bd = desc_codes + b * (L::CODE_BYTES >> 4), sfd = desc_sf + b * (L::SF_BYTES >> 4);
-          const uint32_t at = tmem + L::T_CODES + b * MT * 32;
-          const uint32_t sf_t = tmem + L::T_SF + sfset * L::SF_COLS;  // [V: mt][w], [U: w] scale columns
-          const uint32_t sfu_t = sf_t + MT * W * 4;
+          const uint32_t at = tmem + L::T_CODES + b * 32;
+          const uint32_t sf_t = tmem + L::T_SF + sfset * L::SF_COLS;  // scale columns: V [word], U [word][128 columns]
+          const uint32_t sfu_t = sf_t + W * 4;
           if (elected) {
 #pragma unroll
-            for (int j = 0; j < MT * W; ++j) scales_to_tmem(sf_t + 4 * j, sfd + 32 * j);
+            for (int j = 0; j < W; ++j) scales_to_tmem(sf_t + 4 * j, sfd + 32 * j);
 #pragma unroll
             for (int j = 0; j < W; ++j)
 #pragma unroll
-              for (int h = 0; h < L::NBH; ++h) scales_to_tmem(sfu_t + (j * L::NBH + h) * 4, sfd + 32 * (MT * W + h * W + j));
+              for (int h = 0; h < L::NBH; ++h) scales_to_tmem(sfu_t + (j * L::NBH + h) * 4, sfd + 32 * (W + h * W + j));
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-              if (mt >= mts) continue;
-#pragma unroll
-              for (int s = 0; s < 4; ++s) {  // 64 code steps each; their two scale bytes sit in half (id 0 / 2) of a word
-                const int word = S == 128 ? 0 : s >> 1, id = S == 128 ? (s >> 1) * 2 : (s & 1) * 2;
-                mma_codes(tmem + mt * BN, at + mt * 32 + 8 * s, bd + 2 * s, idesc | ((uint32_t)id << 4) | ((uint32_t)id << 29),
-                          sf_t + (mt * W + word) * 4, sfu_t + word * L::NBH * 4, s > 0 ? 1u : accumulate);
-              }
+            for (int s = 0; s < 4; ++s) {  // 64 code steps each; their two scale bytes sit in half (id 0 / 2) of a word
+              const int word = S == 128 ? 0 : s >> 1, id = S == 128 ? (s >> 1) * 2 : (s & 1) * 2;
+              mma_codes(tmem, at + 8 * s, bd + 2 * s, idesc | ((uint32_t)id << 4) | ((uint32_t)id << 29), sf_t + word * 4,
+                        sfu_t + word * L::NBH * 4, s > 0 ? 1u : accumulate);
             }
             tc_commit(bar_empty + 8 * b);
             if (i + 1 == stages) tc_commit(bar_done);
@@ -597,43 +668,52 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
       }
     }
   } else {
-    // ---- operand warps: 32 rows of V (w < 4 MT) or columns of U each ----------------------------
-    const bool is_v = w < 4 * MT;
-    const int wu = w - 4 * MT;
-    const int row0 = is_v ? 32 * w : 32 * wu;
-    uint8_t* const raw = smem + L::OFF_RAW + w * 4096;
-    const uint32_t raw_s = smem0 + L::OFF_RAW + w * 4096;
-    int4* const rowinfo = reinterpret_cast<int4*>(smem + L::OFF_ROW) + (is_v ? row0 : 0);
+    // ---- operand warps: 32 rows of V (w < 8) or columns of U each, one half of every block ----------
+    const bool is_v = w < 8;
+    const int group = is_v ? w & 3 : (w - 8) % GU;
+    const int half = is_v ? w >> 2 : (w - 8) / GU;
+    const uint32_t raw_s = smem0 + L::OFF_RAW + w * 2 * CT_RAW;
+    int4* const rowinfo = reinterpret_cast<int4*>(smem + L::OFF_ROW) + (is_v ? 32 * w : 0);
+    // first row of V or column of U of this warp in a tile; -1: beyond the operand
+    auto first_row = [&](int tp, int tq) {
+      if (is_v) {
+        const long long r = (long long)tp * CT_ROWS + (int)rank * 128 + 32 * group;
+        return r < prm.P ? (int)r : -1;
+      }
+      const int own = tile_columns(tq) / 2, q = tq * BN + (int)rank * own + 32 * group;
+      return 32 * group < own && q < prm.Q ? q : -1;
+    };
     const bool kmode = is_v ? (cp.v_mode == CT_KVEC || cp.v_mode == CT_KSCL) : (cp.u_mode == CT_KVEC || cp.u_mode == CT_KSCL);
     const int rows = is_v ? cp.rows_v : cp.rows_u, sh = is_v ? cp.sh_v : cp.sh_u;
     const uint32_t row_mask = (uint32_t)rows - 1u;
-    const uint8_t* const tab = reinterpret_cast<const uint8_t*>((is_v ? tab_v : tab_u) + (lane & (REP - 1)));
+    const uint32_t tab = smem0 + L::OFF_TAB + (is_v ? 0 : (cp.rows_v + 1) * CH * REP * 16) + (lane & (REP - 1)) * 16;
     const int tab_chunk = (rows + 1) * REP * 16;
-    // this lane's row in a code stage and its place among the scale words
-    const uint32_t code_t = tmem + L::T_CODES + (w >> 2) * 32 + ((uint32_t)(w & 3) << 21);
-    const uint32_t sf_off = L::OFF_SF + (is_v ? (w >> 2) * W * 512 : (MT + (wu >> 2)) * W * 512) + lane * 16 + ((is_v ? w : wu) & 3) * 4;
+    // this lane's row of V codes in tensor memory, its place among the scale words (U: set for each tile)
+    const uint32_t code_t = tmem + L::T_CODES + ((uint32_t)(w & 3) << 21);
+    uint32_t sf_off = L::OFF_SF + lane * 16 + group * 4;
+    const uint32_t peer_smem = cluster_addr(smem0, rank ^ 1u), peer_full = cluster_addr(bar_full, rank ^ 1u);
+    const uint32_t lead_free = cluster_addr(bar_free, 0);
 
     RowFetch rf;
-    long long ld_at = run_at;
-    int ld_p = 0, ld_q = 0, ld_z = 0, ld_kb = 0, ld_kb1 = 0, ld_buf = 0;
+    rf.k_at = half * CT_HALF;
+    int ld_at = run_at;
+    int ld_p = 0, ld_q = 0, ld_z = 0, ld_kb = 0, ld_kb1 = 0, ld_buf = 0, ld_first = -1;
     auto fetch_next = [&]() {
       if (ld_kb == ld_kb1 && ld_at < run_end) {
         decode_tile(ld_at, ld_p, ld_q, ld_z, ld_kb, ld_kb1);
         ld_at += ld_kb1 - ld_kb;
-        rf.new_tile(cp, is_v, ld_p * BM + row0, rowinfo, lane);
+        ld_first = first_row(ld_p, ld_q);
+        rf.new_tile(cp, is_v, ld_first < 0 ? prm.P : ld_first, rowinfo, lane);
       }
       if (ld_kb < ld_kb1) {
-        if (is_v) {
-          if (ld_p * BM + row0 >= prm.P) {
-          } else if (cp.step_v)
-            rf.step_v(cp, prm.V + (long long)ld_z * prm.v_bs, ld_kb, rowinfo, raw_s + ld_buf * 2048, lane);
-          else
-            rf.fetch_v(cp, prm.V + (long long)ld_z * prm.v_bs, ld_p * BM + row0, ld_kb, rowinfo, raw_s + ld_buf * 2048, lane);
-        } else if (ld_q * BN + row0 < prm.Q) {
-          if (cp.step_u)
-            rf.step_u(cp, prm.U + (long long)ld_z * prm.u_bs, ld_q * BN + row0, ld_kb, raw_s + ld_buf * 2048, lane);
-          else
-            rf.fetch_u(cp, prm.U + (long long)ld_z * prm.u_bs, ld_q * BN + row0, ld_kb, raw_s + ld_buf * 2048, lane);
+        const uint32_t dst = raw_s + ld_buf * CT_RAW;
+        if (ld_first < 0) {
+        } else if (is_v) {
+          if (cp.step_v) rf.step_v(cp, prm.V + (long long)ld_z * prm.v_bs, ld_kb, rowinfo, dst, lane);
+          else rf.fetch_v(cp, prm.V + (long long)ld_z * prm.v_bs, ld_first, ld_kb, rowinfo, dst, lane);
+        } else {
+          if (cp.step_u) rf.step_u(cp, prm.U + (long long)ld_z * prm.u_bs, ld_first, ld_kb, dst, lane);
+          else rf.fetch_u(cp, prm.U + (long long)ld_z * prm.u_bs, ld_first, ld_kb, dst, lane);
         }
         ++ld_kb;
         ld_buf ^= 1;
@@ -641,56 +721,61 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    // Ring position: with a whole number of turns per block the stage buffer and its barriers are constants of
-    // the unrolled loop; otherwise they are counted.
-    constexpr int SPK = C::STAGES_PER_KB;
-    constexpr bool FIXED = SPK % NST == 0;
-    uint32_t b_var = 0, phase = 1, chunk = 0;  // stage buffer (not FIXED), parity of its 'empty' barrier
-    const uint32_t code_base = smem0 + (row0 + lane) * 128;
-    uint32_t code_sw[8];                       // this lane's eight 16-byte places in a stage row (128-byte swizzle)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) code_sw[i] = ((uint32_t)i << 4) ^ ((uint32_t)(lane & 7) << 4);
+    constexpr int SPH = C::STAGES_PER_KB / 2;   // stages this warp makes of a block, then the other warp of its rows as many
+    // Skipping the other warp's stages, a warp may find a barrier SPH + 1 stages behind: this has to be less than one turn
+    // of the ring, or the parity it waits for is that of the turn before.
+    static_assert(SPH < NST, "ring");
+    uint32_t b = 0, phase = 1, chunk = 0;       // stage buffer, parity of its 'empty' barrier
+    auto advance = [&](int n) {
+      b += n;
+      if (b >= NST) {
+        b -= NST;
+        phase ^= 1;
+      }
+    };
+    if (half) advance(SPH);
+    // this lane's row of a stage of U codes, 16-byte place i at (i ^ row & 7) (128-byte swizzle)
+    const uint32_t code_base = smem0 + (32 * group + lane) * 128 + ((uint32_t)(lane & 7) << 4);
     const int grp = w >> 2;
     float* slot = nullptr;  // this thread's place among the parked tiles
-    // One unit of the finished tensor-memory tile plus what earlier chunks of the segment left in the slot.
-    auto load_unit = [&](int i, bool first, float (&v)[16]) {
-      uint32_t r[16];
-      tmem_load16(tmem + ((uint32_t)(w & 3) << 21) + (grp + i * NG) * 16, r);
+    auto read_slot = [&](int i, float (&v)[16]) {
 #pragma unroll
-      for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(r[c]);
-      if (!first) {
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-          if (AMSIM_IN(prm, BUF_WS, slot + (i * 16 + c) * A::NTE, float)) v[c] = __fadd_rn(__ldcg(slot + (i * 16 + c) * A::NTE), v[c]);
-      }
+      for (int c = 0; c < 16; ++c) v[c] = AMSIM_IN(prm, BUF_WS, slot + (i * 16 + c) * A::NTE, float) ? __ldcg(slot + (i * 16 + c) * A::NTE) : 0.f;
     };
     auto park_unit = [&](int i, const float (&v)[16]) {
 #pragma unroll
       for (int c = 0; c < 16; ++c)
         if (AMSIM_IN(prm, BUF_WS, slot + (i * 16 + c) * A::NTE, float)) __stcg(slot + (i * 16 + c) * A::NTE, v[c]);
     };
-    auto begin_drain = [&]() {
+    // Takes this thread's units of a finished chunk out of tensor memory, adds what earlier chunks of the segment
+    // left in the slot (first: nothing) and hands them on; the next chunk's products may begin once all are out.
+    // The tensor core idles meanwhile, so the slot is read a unit ahead, from before the chunk is done.
+    auto take_chunk = [&](bool first, auto&& use) {
+      const int units = (A::UNITS - grp + NG - 1) / NG;
+      float s[16];
+      if (!first) read_slot(0, s);
       wt.wait_warp(bar_done, chunk & 1);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    };
-    auto end_drain = [&]() {
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_free);
-    };
-    // Moves a finished chunk of the segment from tensor memory to the slot and frees it.
-    auto drain = [&](bool first) {
-      if (grp < NG) {
-        begin_drain();
 #pragma unroll 1
-        for (int i = 0; i < UPT; ++i) {
-          if (grp + i * NG >= A::UNITS) break;
-          float v[16];
-          load_unit(i, first, v);
-          park_unit(i, v);
+      for (int i = 0; i < units; ++i) {
+        float v[16];
+        tmem_load16(tmem + ((uint32_t)(w & 3) << 21) + (grp + i * NG) * 16, v);
+        if (i + 1 == units) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(lead_free);
         }
-        end_drain();
+        if (!first) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c) v[c] = __fadd_rn(s[c], v[c]);
+          if (i + 1 < units) read_slot(i + 1, s);
+        }
+        use(i, v);
       }
+    };
+    // Moves a finished chunk of the segment to the slot.
+    auto drain = [&](bool first) {
+      if (grp < NG) take_chunk(first, park_unit);
       ++chunk;
     };
 
@@ -700,40 +785,53 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
       int cp_, cq, cz, kb0, kb1;
       decode_tile(run_at, cp_, cq, cz, kb0, kb1);
       run_at += kb1 - kb0;
-      const bool active = is_v ? cp_ * BM + row0 < prm.P : cq * BN + row0 < prm.Q;
-      slot = prm.ws + ((long long)blockIdx.x * 2 + (kb0 == 0 ? 1 : 0)) * A::SLOT_FLOATS + t;
+      const bool active = first_row(cp_, cq) >= 0;
+      const int own = tile_columns(cq) / 2;
+      const bool sends = !is_v && 32 * group < own;  // (also for columns beyond Q: the other CTA counts on own * 4 * W bytes)
+      if (!is_v) {
+        const int place = (int)rank * (own / 32) + group;  // of the pair's 32-column groups
+        sf_off = L::OFF_SF + (1 + (place >> 2)) * W * 512 + lane * 16 + (place & 3) * 4;
+      }
+      slot = prm.ws + (((long long)pair * 2 + (kb0 == 0 ? 1 : 0)) * 2 + rank) * A::SLOT_FLOATS + t;
       bool pending = false, fresh = true;
-      int since = 0;
+      int ahead = half * SPH;  // own stages of the next chunk start here
       for (int kb = kb0; kb < kb1; ++kb) {
         fetch_next();
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
-        const uint8_t* rb = raw + buf * 2048;
+        const uint32_t rb = raw_s + buf * CT_RAW;
         buf ^= 1;
+        // the next chunk's first stages are made while the last one finishes, as many as the ring holds: a finished
+        // chunk is taken out at once (until then the tensor core idles)
+        if (pending && (ahead + SPH > NST || __all_sync(0xffffffffu, mbar_test(bar_done, chunk & 1)))) {
+          drain(fresh);
+          fresh = pending = false;
+        }
+        ahead += C::STAGES_PER_KB;
 #pragma unroll
-        for (int j = 0; j < SPK; ++j) {
-          if (j == NST % SPK && pending && since == NST - NST % SPK) {  // the next chunk's first stages are made while the last one finishes
-            drain(fresh);
-            fresh = pending = false;
-          }
-          const uint32_t b = FIXED ? (uint32_t)(j % NST) : b_var;
+        for (int j = 0; j < SPH; ++j) {
           uint32_t x[KS];
           uint4 q[8];
-          if (active) {
+          if (!active) {
+#pragma unroll
+            for (int e = 0; e < KS; ++e) x[e] = 0;
+          } else {
             if (kmode) {
+              const uint32_t row = rb + lane * 32;
+              const int flip = (lane >> 2) & 1;
               if (KS == 2) {
-                const uint2 v = *reinterpret_cast<const uint2*>(rb + lane * 64 + (((j >> 1) ^ ((lane >> 1) & 3)) << 4) + (j & 1) * 8);
+                const uint2 v = lds64(row + (((j >> 1) ^ flip) << 4) + (j & 1) * 8);
                 x[0] = v.x; x[1] = v.y;
               } else {
 #pragma unroll
                 for (int i = 0; i < KS / 4; ++i) {
-                  const uint4 v = *reinterpret_cast<const uint4*>(rb + lane * 64 + (((j * (KS / 4) + i) ^ ((lane >> 1) & 3)) << 4));
+                  const uint4 v = lds128(row + (((j * (KS / 4) + i) ^ flip) << 4));
                   x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[(4 * i + 3) % KS] = v.w;
                 }
               }
             } else {
 #pragma unroll
-              for (int i = 0; i < KS; ++i) x[i] = *reinterpret_cast<const uint32_t*>(rb + (j * KS + i) * 128 + lane * 4);
+              for (int i = 0; i < KS; ++i) x[i] = lds32(rb + (j * KS + i) * 128 + lane * 4);
             }
             // all eight 16-byte pieces are read before the first is stored (the compiler cannot tell that the
             // stage and the table do not overlap), and before the wait for the stage
@@ -741,9 +839,9 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
             for (int e = 0; e < KS; ++e) {
               // zero and denormal elements take the table's zero row: their products are exactly 0
               const uint32_t idx = (x[e] & 0x7F800000u) ? ((x[e] >> sh) & row_mask) : (uint32_t)rows;
-              const uint8_t* src = tab + idx * (REP * 16);
+              const uint32_t src = tab + idx * (REP * 16);
 #pragma unroll
-              for (int c = 0; c < CH; ++c) q[e * CH + c] = *reinterpret_cast<const uint4*>(src + c * tab_chunk);
+              for (int c = 0; c < CH; ++c) q[e * CH + c] = lds128(src + c * tab_chunk);
             }
           }
           wt.wait_warp(bar_empty + 8 * b, phase);
@@ -755,42 +853,47 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
               q[i].x ^= sign; q[i].y ^= sign; q[i].z ^= sign; q[i].w ^= sign;
             }
             if (is_v) {
-              tmem_store32(code_t + b * MT * 32, q);
+              tmem_store32(code_t + b * 32, q);
               asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             } else {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) sts128(code_base + code_sw[i] + b * L::CODE_BYTES, q[i]);
+              for (int i = 0; i < 8; ++i) sts128((code_base + b * L::CODE_BYTES) ^ ((uint32_t)i << 4), q[i]);
             }
-            // scale bytes = exponent fields; one 32-bit word covers two matrix instructions
-            uint8_t* const sfp = smem + sf_off + b * L::SF_BYTES;
+          }
+          // scale bytes = exponent fields; one 32-bit word covers two matrix instructions
+          if (active || sends) {
+            uint32_t sf[W];
             if (S == 64) {
-              *reinterpret_cast<uint32_t*>(sfp) = __byte_perm(x[0] << 1, x[1] << 1, 0x7733);
-              *reinterpret_cast<uint32_t*>(sfp + 512) = __byte_perm(x[2 % KS] << 1, x[3 % KS] << 1, 0x7733);
+              sf[0] = __byte_perm(x[0] << 1, x[1] << 1, 0x7733);
+              sf[W - 1] = __byte_perm(x[2 % KS] << 1, x[3 % KS] << 1, 0x7733);
             } else if (S == 128) {
-              *reinterpret_cast<uint32_t*>(sfp) = __byte_perm(x[0] << 1, x[1] << 1, 0x7733);
+              sf[0] = __byte_perm(x[0] << 1, x[1] << 1, 0x7733);
             } else {
 #pragma unroll
-              for (int i = 0; i < 2; ++i) {
+              for (int i = 0; i < W; ++i) {
                 const uint32_t lo = __byte_perm(x[(4 * i) % KS] << 1, x[(4 * i + 1) % KS] << 1, 0x0073);
                 const uint32_t hi = __byte_perm(x[(4 * i + 2) % KS] << 1, x[(4 * i + 3) % KS] << 1, 0x0073);
-                *reinterpret_cast<uint32_t*>(sfp + 512 * i) = __byte_perm(lo, hi, 0x5410);
+                sf[i] = __byte_perm(lo, hi, 0x5410);
               }
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            const uint32_t sf_at = sf_off + b * L::SF_BYTES;
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+              sts32(smem0 + sf_at + 512 * i, sf[i]);
+              if (sends) st_async_remote(peer_smem + sf_at + 512 * i, sf[i], peer_full + 8 * b);  // both CTAs need every column's scales
+            }
           }
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar_full + 8 * b);
-          if (FIXED) {
-            if ((j + 1) % NST == 0) phase ^= 1;
-          } else if (++b_var == NST) {
-            b_var = 0;
-            phase ^= 1;
+          if (lane == 0) {
+            if (is_v && group == 0) mbar_arrive_expect(bar_full + 8 * b, own * 4 * W);
+            else mbar_arrive(bar_full + 8 * b);
           }
+          advance(1);
         }
-        since += SPK;
+        advance(SPH);
         if ((kb - kb0 + 1) % CT_CHUNK == 0 && kb + 1 < kb1) {
           pending = true;
-          since = 0;
+          ahead = half * SPH;
         }
       }
       if (pending) {
@@ -804,9 +907,9 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
         const bool shared_tile = kb0 != 0 || kb1 != nkb_all;
         float* __restrict__ Og = prm.O + (long long)cz * prm.o_bs;
         const bool vec_out = prm.o_sq == 1 && (prm.o_sp & 3) == 0 && (prm.o_bs & 3) == 0 && ((reinterpret_cast<uintptr_t>(prm.O) & 15) == 0);
-        auto write_unit = [&](int i, float (&v)[16]) {
+        auto write_unit = [&](int i, const float (&v)[16]) {
           const int u = grp + i * NG;
-          const int pg = cp_ * BM + (u / (BN / 16)) * 128 + (w & 3) * 32 + lane, q0 = cq * BN + (u % (BN / 16)) * 16;
+          const int pg = cp_ * CT_ROWS + (int)rank * 128 + (w & 3) * 32 + lane, q0 = cq * BN + u * 16;
           if (pg >= prm.P || q0 >= prm.Q) return;
           long long row = pg;
           if (prm.o_strided) {
@@ -825,31 +928,27 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
             store_out4(prm, orow, q0 + 4 * c4, o, vec_out);
           }
         };
-        begin_drain();
-#pragma unroll 1
-        for (int i = 0; i < UPT; ++i) {
-          if (grp + i * NG >= A::UNITS) break;
-          float v[16];
-          load_unit(i, fresh, v);
+        take_chunk(fresh, [&](int i, const float (&v)[16]) {
           if (shared_tile) park_unit(i, v);
           else write_unit(i, v);
-        }
-        end_drain();
+        });
         if (shared_tile) {
-          // a tile shared between runs: count in; the last sharer adds the parked tiles in CTA order
+          // a tile shared between runs: count in; the last sharer adds the parked tiles in the order of the runs
+          // (each CTA of the pair its own rows, counted apart)
           __threadfence();
           asm volatile("bar.sync 1, %0;" ::"r"(A::NTE) : "memory");
           const long long first = tile * nkb_all, last = first + nkb_all;
-          long long c0 = first * prm.sk_grid / prm.sk_iters;
+          int c0 = (int)(first * prm.sk_grid / prm.sk_iters);
           while (c0 > 0 && balanced_begin(c0, prm.sk_iters, prm.sk_grid) > first) --c0;
           while (balanced_begin(c0 + 1, prm.sk_iters, prm.sk_grid) <= first) ++c0;
-          long long c1 = (last - 1) * prm.sk_grid / prm.sk_iters;
+          int c1 = (int)((last - 1) * prm.sk_grid / prm.sk_iters);
           while (c1 > 0 && balanced_begin(c1, prm.sk_iters, prm.sk_grid) > last - 1) --c1;
           while (balanced_begin(c1 + 1, prm.sk_iters, prm.sk_grid) <= last - 1) ++c1;
           if (t == 0) {
-            const int arrived = AMSIM_IN(prm, BUF_WS, prm.sk_count + tile, int) ? atomicAdd(prm.sk_count + tile, 1) : 0;
-            flag_s = arrived == (int)(c1 - c0);
-            if (arrived == (int)(c1 - c0) && AMSIM_IN(prm, BUF_WS, prm.sk_count + tile, int)) prm.sk_count[tile] = 0;
+            int* const count = prm.sk_count + 2 * tile + rank;
+            const int arrived = AMSIM_IN(prm, BUF_WS, count, int) ? atomicAdd(count, 1) : 0;
+            flag_s = arrived == c1 - c0;
+            if (arrived == c1 - c0 && AMSIM_IN(prm, BUF_WS, count, int)) *count = 0;
           }
           asm volatile("bar.sync 1, %0;" ::"r"(A::NTE) : "memory");
           const bool completes = flag_s != 0;
@@ -862,12 +961,27 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
               float v[16];
 #pragma unroll
               for (int c = 0; c < 16; ++c) v[c] = 0.f;
-              for (long long cta = c0; cta <= c1; ++cta) {
-                const long long bg = balanced_begin(cta, prm.sk_iters, prm.sk_grid);
-                const float* src = prm.ws + (cta * 2 + (bg <= first ? 1 : 0)) * A::SLOT_FLOATS + t;
+              // the sharers' tiles four at a time: 16 loads in flight (one tile after the other took a round trip to L2 each)
+              for (int run = c0; run <= c1; run += 4) {
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                  if (AMSIM_IN(prm, BUF_WS, src + (i * 16 + c) * A::NTE, float)) v[c] = __fadd_rn(v[c], __ldcg(src + (i * 16 + c) * A::NTE));
+                for (int h = 0; h < 4; ++h) {
+                  float part[4][4];
+#pragma unroll
+                  for (int r = 0; r < 4; ++r) {
+                    const bool first_run = balanced_begin(run + r, prm.sk_iters, prm.sk_grid) <= first;
+                    const float* src = prm.ws + (((long long)(run + r) * 2 + (first_run ? 1 : 0)) * 2 + rank) * A::SLOT_FLOATS + t;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                      const float* at = src + (i * 16 + h * 4 + c) * A::NTE;
+                      part[r][c] = run + r <= c1 && AMSIM_IN(prm, BUF_WS, at, float) ? __ldcg(at) : 0.f;
+                    }
+                  }
+#pragma unroll
+                  for (int r = 0; r < 4; ++r)
+                    if (run + r <= c1)
+#pragma unroll
+                      for (int c = 0; c < 4; ++c) v[h * 4 + c] = __fadd_rn(v[h * 4 + c], part[r][c]);
+                }
               }
               write_unit(i, v);
             }
@@ -880,7 +994,8 @@ __global__ void __launch_bounds__(CodeSmem<S, MT, BN>::NT, 1) code_gemm(const __
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (w == NW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+  cluster_barrier();  // neither CTA leaves while the other may still reach its shared or tensor memory
+  if (w == NW) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
 
 }  // namespace amsim

@@ -7,10 +7,10 @@ namespace amsim {
 
 struct CodeParams;
 
-// Tile shapes of code_gemm: 0 = 128 x 256, 1 = 256 x 128, 2 = 256 x 64 (rows of V x columns of U).
+// Tile shapes of code_gemm: 0 = 256 x 256, 1 = 256 x 128, 2 = 256 x 64 (rows of V x columns of U of a CTA pair).
 struct CodeTile {
   int bm, bn;
-  size_t slot_bytes;  // one parked tile of register accumulators
+  size_t slot_bytes;  // one parked tile (both CTAs' halves)
 };
 CodeTile code_tile(int shape);
 cudaError_t code_gemm_launch(cudaStream_t st, const CodeParams& cp, int shape, int device);
