@@ -29,8 +29,8 @@
 // operand words fetched from shared memory share that path (the lane operand
 // is ONE packed word per element; the uniform operand is kept as two words,
 // sign+exponent and table row, because unpacking it in the loop costs more
-// issue slots than the second broadcast load costs wavefronts).  Tensor cores
-// cannot be used: no product is a hardware multiply.
+// issue slots than the second broadcast load costs wavefronts).  Large fast-mode
+// products over tables that factor run on the tensor cores (amsim_codes.cuh).
 //
 // Besides the plain grid (one CTA per 128 x 64 tile) gather_gemm has a balanced
 // mode (equal runs of (tile, reduction block) pairs over exactly the resident
