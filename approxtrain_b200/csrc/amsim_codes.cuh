@@ -504,16 +504,20 @@ struct RowFetch {
   }
 };
 
-// Writes 4 consecutive columns of one output row through the epilogue (see store_out_tile).
+// The epilogue of one output of column q (see store_out_tile).
+__device__ __forceinline__ float finish_out(const Params& prm, float o, int q) {
+  if (prm.has_alpha) o = __fmul_rn(o, prm.alpha);
+  if (prm.scale != nullptr) o = __fmul_rn(o, __ldg(prm.scale + q));
+  if (prm.bias != nullptr) o = __fadd_rn(o, __ldg(prm.bias + q));
+  return prm.relu && o < 0.f ? 0.f : o;
+}
+
+// Writes 4 consecutive columns of one output row through the epilogue.
 __device__ __forceinline__ void store_out4(const Params& prm, float* __restrict__ orow, int qg, float (&o)[4], bool vec_out) {
   if (prm.bias != nullptr || prm.relu || prm.scale != nullptr || prm.has_alpha) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (prm.has_alpha) o[r] = __fmul_rn(o[r], prm.alpha);
-      if (prm.scale != nullptr && qg + r < prm.Q) o[r] = __fmul_rn(o[r], __ldg(prm.scale + qg + r));
-      if (prm.bias != nullptr && qg + r < prm.Q) o[r] = __fadd_rn(o[r], __ldg(prm.bias + qg + r));
-      if (prm.relu) o[r] = o[r] < 0.f ? 0.f : o[r];
-    }
+    for (int r = 0; r < 4; ++r)
+      if (qg + r < prm.Q) o[r] = finish_out(prm, o[r], qg + r);
   }
   if (vec_out && qg + 3 < prm.Q) {
     if (AMSIM_IN(prm, BUF_O, orow + qg, float4)) *reinterpret_cast<float4*>(orow + qg) = make_float4(o[0], o[1], o[2], o[3]);
@@ -522,6 +526,81 @@ __device__ __forceinline__ void store_out4(const Params& prm, float* __restrict_
     for (int r = 0; r < 4; ++r)
       if (qg + r < prm.Q && AMSIM_IN(prm, BUF_O, orow + (long long)(qg + r) * prm.o_sq, float)) orow[(long long)(qg + r) * prm.o_sq] = o[r];
   }
+}
+
+// First element of output row pg of batch z.
+__device__ __forceinline__ float* out_row(const Params& prm, int z, int pg) {
+  const Gather& g = prm.g;
+  long long row = pg;
+  if (prm.o_strided) {
+    const uint32_t n = fdiv((uint32_t)pg, g.d_img);
+    const uint32_t rem = (uint32_t)pg - n * (uint32_t)(g.PH * g.PW);
+    const uint32_t yy = fdiv(rem, g.d_pw);
+    const uint32_t xx = rem - yy * (uint32_t)g.PW;
+    row = ((long long)n * prm.o_h + (long long)yy * prm.o_sh + prm.o_a) * prm.o_w + (long long)xx * prm.o_sw + prm.o_b;
+  }
+  return prm.O + (long long)z * prm.o_bs + row * prm.o_sp;
+}
+
+// Recomputes those of 16 outputs (row pg of batch z, columns q0..) that a tile has left as NaN, as the table kernels'
+// chain over the whole reduction.  An accumulator holds out / unit (1 / unit is up to 64), so sums from 2^122 on are
+// infinite there, and nothing makes them finite again; FP32 holds them up to 2^128.  Operands with exponent field 255
+// give NaN for every output they take part in.  A chain that has become NaN ends.
+static __device__ __noinline__ void repair_outputs(const CodeParams& cp, int z, int pg, int q0) {
+  const Params& prm = cp.prm;
+  const Gather& g = prm.g;
+  const float* const Vg = prm.V + (long long)z * prm.v_bs;
+  const float* const Ug = prm.U + (long long)z * prm.u_bs;
+  float* const orow = out_row(prm, z, pg);
+  float s[16];
+  uint32_t todo = 0;
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    const float* const at = orow + (long long)(q0 + c) * prm.o_sq;
+    const float was = q0 + c < prm.Q && AMSIM_IN(prm, BUF_O, at, float) ? *at : 0.f;
+    s[c] = 0.f;
+    if (was != was) todo |= 1u << c;
+  }
+  const uint32_t redo = todo;
+  for (int k = 0; k < prm.K && todo; ++k) {
+    const float* src = Vg;
+    bool ok = true;
+    if (!cp.fgrad && prm.v_trans) {
+      src += (long long)k * prm.v_ld + pg;
+    } else {  // (filter gradient: pg is a filter element and k a grid position; otherwise the other way round)
+      const uint32_t pix = (uint32_t)(cp.fgrad ? k : pg), el = (uint32_t)(cp.fgrad ? pg : k);
+      const uint32_t n = fdiv(pix, g.d_img);
+      const uint32_t rem = pix - n * (uint32_t)(g.PH * g.PW);
+      const uint32_t a = fdiv(rem, g.d_pw);
+      const uint32_t b = rem - a * (uint32_t)g.PW;
+      const uint32_t tap = fdiv(el, g.d_sc);
+      const int ch = (int)(el - tap * (uint32_t)g.SC);
+      const int kh = (int)fdiv(tap, g.d_kw), kw = (int)tap - kh * g.KW;
+      const int u = (int)a * g.ps_h - g.off_t + kh, v = (int)b * g.ps_w - g.off_l + kw;
+      ok = (unsigned)u < (unsigned)g.lim_h && (unsigned)v < (unsigned)g.lim_w;
+      if (ok) src += (long long)n * ((long long)g.SH * g.SW * g.SC) + ((long long)(u * g.SW + v) * g.SC + ch);
+    }
+    ok = ok && AMSIM_IN(prm, BUF_V, src, float);
+    const uint32_t vb = ok ? __float_as_uint(__ldg(src)) : 0u;
+    const uint32_t iv = (vb >> (23 - prm.m)) & prm.cmask;
+    const long long u_at = RowFetch::u_offset(cp, k);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      if (!((todo >> c) & 1u)) continue;
+      const float* const us = Ug + u_at + (long long)(q0 + c) * prm.u_sq;
+      const uint32_t ub = AMSIM_IN(prm, BUF_U, us, float) ? __float_as_uint(__ldg(us)) : 0u;
+      if ((vb & 0x7F800000u) == 0x7F800000u || (ub & 0x7F800000u) == 0x7F800000u) {
+        s[c] = __uint_as_float(0x7FFFFFFFu);
+      } else if (vb & 0x7F800000u) {  // as in mac_step
+        const uint32_t e = (uint32_t)__ldg(prm.lut + ((((ub >> (23 - prm.m)) & prm.cmask) << prm.m) | iv)) * prm.mult;
+        s[c] = __fmaf_rn(__uint_as_float(ub & 0xFF800000u), __uint_as_float(e + (vb & 0xFF800000u)), s[c]);
+      }
+      if (s[c] != s[c]) todo &= ~(1u << c);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 16; ++c)
+    if ((redo >> c) & 1u) orow[(long long)(q0 + c) * prm.o_sq] = finish_out(prm, s[c], q0 + c);
 }
 
 // Share of a thread in draining and writing a tile: 16-column units u = g, g + NG, ... of the tile (g = warp / 4), of
@@ -546,6 +625,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
   __shared__ uint64_t bars[3 * NST + 2];
   __shared__ uint32_t tmem_holder;
   __shared__ int flag_s;
+  __shared__ int odd_s;    // outputs that are not finite have been written (repair_outputs)
+  __shared__ int wrote_s;  // this CTA has written its rows of the run's first (1) or last (2) tile, shared with other runs
   const Params& prm = cp.prm;
   const Gather& g = prm.g;
   const uint32_t smem0 = (smem_addr(smem_raw) + 1023u) & ~1023u;
@@ -567,6 +648,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
     mbar_init(bar_done, 1);
     mbar_init(bar_free, 2 * 4 * NG);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    odd_s = wrote_s = 0;
   }
   if (w == NW) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_addr(&tmem_holder)) : "memory");
@@ -905,28 +987,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
       if (grp < NG) {
         const long long tile = ((long long)cz * prm.sk_ptiles + cp_) * prm.sk_qtiles + cq;
         const bool shared_tile = kb0 != 0 || kb1 != nkb_all;
-        float* __restrict__ Og = prm.O + (long long)cz * prm.o_bs;
         const bool vec_out = prm.o_sq == 1 && (prm.o_sp & 3) == 0 && (prm.o_bs & 3) == 0 && ((reinterpret_cast<uintptr_t>(prm.O) & 15) == 0);
         auto write_unit = [&](int i, const float (&v)[16]) {
           const int u = grp + i * NG;
           const int pg = cp_ * CT_ROWS + (int)rank * 128 + (w & 3) * 32 + lane, q0 = cq * BN + u * 16;
           if (pg >= prm.P || q0 >= prm.Q) return;
-          long long row = pg;
-          if (prm.o_strided) {
-            const uint32_t n = fdiv((uint32_t)pg, g.d_img);
-            const uint32_t rem = (uint32_t)pg - n * (uint32_t)(g.PH * g.PW);
-            const uint32_t yy = fdiv(rem, g.d_pw);
-            const uint32_t xx = rem - yy * (uint32_t)g.PW;
-            row = ((long long)n * prm.o_h + (long long)yy * prm.o_sh + prm.o_a) * prm.o_w + (long long)xx * prm.o_sw + prm.o_b;
-          }
-          float* orow = Og + row * prm.o_sp;
+          float* const orow = out_row(prm, cz, pg);
+          bool finite = true;
 #pragma unroll
           for (int c4 = 0; c4 < 4; ++c4) {
             float o[4];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) o[r] = __fmul_rn(v[4 * c4 + r], cp.unit);
+            for (int r = 0; r < 4; ++r) {
+              o[r] = __fmul_rn(v[4 * c4 + r], cp.unit);
+              const bool odd = (__float_as_uint(o[r]) & 0x7F800000u) == 0x7F800000u;
+              if (odd) o[r] = __uint_as_float(0x7FFFFFFFu);  // (stays NaN through the epilogue)
+              finite = finite && !odd;
+            }
             store_out4(prm, orow, q0 + 4 * c4, o, vec_out);
           }
+          if (!finite) odd_s = 1;
         };
         take_chunk(fresh, [&](int i, const float (&v)[16]) {
           if (shared_tile) park_unit(i, v);
@@ -952,6 +1032,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
           }
           asm volatile("bar.sync 1, %0;" ::"r"(A::NTE) : "memory");
           const bool completes = flag_s != 0;
+          if (completes && t == 0) wrote_s |= kb0 == 0 ? 2 : 1;
           asm volatile("bar.sync 1, %0;" ::"r"(A::NTE) : "memory");
           if (completes) {
             __threadfence();
@@ -994,6 +1075,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (odd_s && w < 4 * NG) {  // each thread looks its own outputs over
+    run_at = (int)balanced_begin(pair, prm.sk_iters, prm.sk_grid);
+    while (run_at < run_end) {
+      int tp, tq, tz, kb0, kb1;
+      decode_tile(run_at, tp, tq, tz, kb0, kb1);
+      run_at += kb1 - kb0;
+      const int pg = tp * CT_ROWS + (int)rank * 128 + (w & 3) * 32 + lane;
+      const bool wrote = (kb0 == 0 && kb1 == nkb_all) || (wrote_s & (kb0 == 0 ? 2 : 1));
+      if (!wrote || pg >= prm.P) continue;
+      for (int u = w >> 2; u < A::UNITS && tq * BN + u * 16 < prm.Q; u += NG) repair_outputs(cp, tz, pg, tq * BN + u * 16);
+    }
+  }
   cluster_barrier();  // neither CTA leaves while the other may still reach its shared or tensor memory
   if (w == NW) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }

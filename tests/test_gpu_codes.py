@@ -71,6 +71,77 @@ def test_matmuls(forced, lut, m, k, n, ta, tb):
     _close(f(False), f(True))
 
 
+def _on(forced, codes, f):
+    os.environ["AMSIM_CODES"] = str(codes)
+    forced.lib.amsim_debug_reload_env()
+    return f()
+
+
+def _same_as_table_kernels(forced, f):
+    """Not finite where the table kernels' result is not, in the same way, and close elsewhere."""
+    got, want = _on(forced, 1, f), _on(forced, 0, f)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(torch.isinf(got), torch.isinf(want))
+    finite = torch.isfinite(want)
+    assert finite.any()
+    _close(got[finite], want[finite])
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7", "MIT_5", "MBM_5"])
+@pytest.mark.parametrize("e", [121, 123, 125, 127])
+def test_products_up_to_the_largest_float(forced, lut, e):
+    """Products of 2^e and their cancelling sums: FP32 holds them, accumulators in units of the table's step do not."""
+    from approxtrain_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(e)
+    x, w = torch.randn(300, 130, generator=g, device="cuda"), torch.randn(130, 200, generator=g, device="cuda")
+    big = 2.0 ** (e // 2)
+    x[5:40, 7], w[7, 3:90] = 2.0 ** (e - e // 2), big
+    _same_as_table_kernels(forced, lambda: ops.denseam(x, w, lut_path(lut)))
+    w[3, 3:90], x[5:40, 3] = -big, 2.0 ** (e - e // 2)      # the sum returns to ordinary size
+    f = lambda: ops.denseam(x, w, lut_path(lut))  # noqa: E731
+    got, want = _on(forced, 1, f), _on(forced, 0, f)
+    assert torch.isfinite(want).all()
+    assert torch.equal(got[5:40, 3:90], want[5:40, 3:90]) or rel_l2(got[5:40, 3:90].cpu().numpy(), want[5:40, 3:90].cpu().numpy()) <= 1e-5
+    assert torch.isfinite(got).all()
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7"])
+@pytest.mark.parametrize("shape", [(2, 9, 13, 16, 3, 3, 65, 1, "SAME"), (3, 11, 7, 8, 3, 3, 129, 2, "SAME"), (1, 30, 30, 3, 7, 7, 64, 2, "VALID"),
+                                   (2, 14, 14, 64, 1, 1, 300, 1, "VALID")])
+def test_huge_operands_in_every_direction(forced, lut, shape):
+    """Sums between 2^122 and 2^128, and products beyond."""
+    from approxtrain_b200 import ops
+    n, h, w, c, kh, kw, k, s, pad = shape
+    g = torch.Generator(device="cuda").manual_seed(h + k)
+    kw_ = dict(strides=s, padding=pad, mant_mul_lut=lut_path(lut))
+    x, wt = torch.randn(n, h, w, c, generator=g, device="cuda"), torch.randn(kh, kw, c, k, generator=g, device="cuda")
+    x[0, 3, 4, 1], x[0, 5, 5, 2], x[n - 1, 6, 2, 0] = 2.0 ** 100, -2.0 ** 62, 2.0 ** 63
+    wt[0, 0, 1, 5], wt[0, 0, 2, 9], wt[kh - 1, 0, 0, 7] = 2.0 ** 25, 2.0 ** 63, -2.0 ** 61
+    _same_as_table_kernels(forced, lambda: ops.convam(x, wt, **kw_))
+    b, sc = torch.randn(k, generator=g, device="cuda"), torch.rand(k, generator=g, device="cuda") - 0.5
+    _same_as_table_kernels(forced, lambda: ops.convam_bias_act(x, wt, b, activation="relu", scale=sc, **kw_))
+    dy = torch.randn(ops.convam(x, wt, **kw_).shape, generator=g, device="cuda")
+    dy[0, 2, 1, 5], dy[0, 1, 2, 9], dy[0, 3, 3, 7] = 2.0 ** 99, 2.0 ** 61, 2.0 ** 62
+    _same_as_table_kernels(forced, lambda: ops.convam_input_grad(x.shape, wt, dy, **kw_))
+    _same_as_table_kernels(forced, lambda: ops.convam_filter_grad(wt.shape, x, dy, **kw_))
+    if kh == 1:
+        a, b = x[0, :, :, :].reshape(-1, c).t().contiguous(), wt[0, 0]
+        _same_as_table_kernels(forced, lambda: ops.matmulam(a, b, transpose_a=True, alpha=0.5, mant_mul_lut=lut_path(lut)))
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7"])
+def test_a_non_finite_operand_makes_its_outputs_nan_and_no_others(forced, lut):
+    from approxtrain_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x, w = torch.randn(700, 300, generator=g, device="cuda"), torch.randn(300, 200, generator=g, device="cuda")
+    clean = ops.denseam(x, w, lut_path(lut))
+    x[3, 7], x[600, 299], w[5, 11], w[6, 190] = float("inf"), float("nan"), -float("inf"), float("nan")
+    y = ops.denseam(x, w, lut_path(lut))
+    bad = torch.zeros(700, 200, dtype=torch.bool, device="cuda")
+    bad[3], bad[600], bad[:, 11], bad[:, 190] = True, True, True, True
+    assert torch.equal(torch.isnan(y), bad) and torch.equal(y[~bad], clean[~bad])
+
+
 def test_zeros_give_zero_and_non_finite_values_stay_visible(forced):
     from approxtrain_b200 import ops
     p = lut_path("MBM_7")
