@@ -667,7 +667,7 @@ int code_stuck_address(int device, unsigned** out) {
 }
 
 struct CodePlan {
-  int use = 0, shape = 0;
+  int use = 0, shape = 0, chunk = 1;
   long long tiles = 0, iters = 0;
   int grid = 0;              // CTA pairs
   size_t slot_bytes = 0;     // parked tiles of the whole launch
@@ -683,16 +683,32 @@ struct CodeTraits {
 // The traits for which the path is taken most readily: the *_workspace functions do not know the table.
 constexpr CodeTraits kCodeTraitsAny = {32, false, true, false};
 
+// 16-step blocks that one accumulator in tensor memory takes before its sum goes on in FP32.  Its adds truncate, which costs
+// in proportion to their number, where one FP32 chain's rounding grows with the square root of its length: the shorter the
+// reduction, the shorter the chunk.  Errors against 64 bits (normal operands; table kernels / 16 / 32 / 64 / 128 steps):
+// MBM_7, K 128 1.43 / 1.46 / 1.54 / 1.68 / 1.77e-8, K 256 2.25 / 2.14 / 2.13 / 2.22 / 2.44e-8, K 512 3.36 / 3.16 / 3.10 /
+// 3.06 / 3.22e-8; MIT_7, K 256 2.37 / 2.24 / 2.26 / 2.45 / 2.86e-8, K 576 3.43 / 3.33 / 3.35 / 3.47 / 3.68e-8, K 2048 6.84 /
+// 6.20 / 6.08 / 5.95 / 5.88e-8.  A chunk of a 256-column tile that is taken out costs a pair 4 to 6 us.
+int code_steps(int K, int slots) {
+  if (slots == 128) return K < 256 ? 1 : K < 512 ? 2 : K < 2048 ? 4 : 8;
+  return K < 256 ? 1 : K < 512 ? 4 : 8;
+}
+// Shorter reductions stay on the table kernels: at K 64 (MIT_7, ordinary operands) 5.3e-9 there, 6.2e-9 here; MBM_7 4.8e-9
+// on both.
+constexpr int code_least_k(int slots) { return slots == 64 ? 64 : 128; }
+
 // Microseconds of one launch on either path, fitted to 75 timed launches (1e6 to 9e9 products, MBM_7, MIT_7 and
-// MIT_5, B200).  Tensor cores: a fixed part, the 16-step blocks of one CTA pair (2.6 / 1.8 / 1.45 us for 256 / 128 /
-// 64 columns and 64 slots), and the parked tiles that the last pair to finish a shared tile adds up.  Table kernels:
-// 165 us per 1e9 lookups, 105 us per 1e9 additive products, and a part that long reductions over few tiles add.
+// MIT_5, B200).  Tensor cores: a fixed part, the 16-step blocks of one CTA pair (2.1 / 1.58 / 1.31 us for 256 / 128 /
+// 64 columns and 64 slots), the partial tiles that go through scratch after every chunk, and the parked tiles that the
+// last pair to finish a shared tile adds up.  Table kernels: 165 us per 1e9 lookups, 105 us per 1e9 additive products,
+// and a part that long reductions over few tiles add.
 // Examples (table kernels / this path): 8192 x 512 x 128, MBM_7 110 / 47 us, MIT_7 78 / 70 us; 784 x 1152 x 128,
 // MBM_7 72 / 51 us; 1024 x 512 x 256, MIT_7 39 / 59 us.
-constexpr double kCodeBlockUs[3] = {2.6, 1.8, 1.45}, kCodeShareUs[3] = {2.2, 1.7, 1.0};
+constexpr double kCodeBlockUs[3] = {2.1, 1.58, 1.31}, kCodeDrainUs[3] = {4.0, 1.9, 1.2}, kCodeShareUs[3] = {2.2, 1.7, 1.0};
 double code_us(const CodePlan& f, const CodeTraits& t) {
   const double block = kCodeBlockUs[f.shape] * (t.slots == 128 ? 1.9 : t.slots == 32 ? 0.85 : 1.0) * (t.scalar ? 1.4 : 1.0);
-  return 16 + ((double)f.iters / f.grid + 2) * block + ((double)f.grid / f.tiles + 1) * kCodeShareUs[f.shape];
+  const double blocks = (double)f.iters / f.grid;
+  return 16 + (blocks + 2) * block + blocks / f.chunk * kCodeDrainUs[f.shape] + ((double)f.grid / f.tiles + 1) * kCodeShareUs[f.shape];
 }
 double table_us(double products, int K, const CodeTraits& t) {
   const double wide = (t.additive ? 24 + 105e-9 * products : 22 + 165e-9 * products) * (t.scalar ? 1.2 : 1.0);
@@ -707,8 +723,11 @@ CodePlan plan_codes(int P, int Q, int K, int batch, int sms, const CodeTraits& t
   const Switches& w = sw();
   const bool picked = w.balanced >= 0 || w.force_ksplit >= 0 || w.no_qsplit || w.no_uvec || w.no_wgrad_swap || w.thin_fast >= 0 || w.wide >= 0;
   if (w.codes == 0 || (w.codes < 0 && picked) || P <= 0 || Q <= 0 || K <= 0 || batch <= 0) return f;
-  f.shape = Q > 128 ? 0 : Q > 64 ? 1 : 2;
+  // (short chunks of 256 columns cost more than the narrower tile: 1x1 256 -> 512 with 2-block chunks 817 us, 128 columns 730)
+  const int steps = code_steps(K, t.slots);
+  f.shape = Q > 128 && steps >= 4 ? 0 : Q > 64 ? 1 : 2;
   const CodeTile tile = code_tile(f.shape);
+  f.chunk = steps * tile.accumulators;
   const long long pt = ((long long)P + tile.bm - 1) / tile.bm, qt = ((long long)Q + tile.bn - 1) / tile.bn;
   f.tiles = pt * qt * batch;
   f.iters = f.tiles * (((long long)K + CT_KB - 1) / CT_KB);
@@ -723,7 +742,7 @@ CodePlan plan_codes(int P, int Q, int K, int batch, int sms, const CodeTraits& t
   // its next product, so a last-bit change of the scores shows as 2e-3 of the result's root mean square there; and a
   // tile's 256 rows are of one product (512 of 128 x 128 x 64: MIT_7 65 / 137 us, MBM_7 109 / 88 us).
   const double products = (double)P * Q * K * batch;
-  if (w.codes < 0 && (batch > 1 || products < 1e8 || code_us(f, t) > 0.95 * table_us(products, K, t))) return f;
+  if (w.codes < 0 && (batch > 1 || products < 1e8 || K < code_least_k(t.slots) || code_us(f, t) > 0.95 * table_us(products, K, t))) return f;
   f.slot_bytes = (size_t)f.grid * 2 * tile.slot_bytes;
   f.counter_bytes = ((size_t)f.tiles * 2 * sizeof(int) + 255) / 256 * 256;
   f.use = 1;
@@ -745,6 +764,7 @@ void code_params(CodeParams& c, const Params& p, const CodePlan& f, bool fgrad) 
   c.sh_u = p.ct_sh_u;
   c.unit = p.ct_unit;
   c.fgrad = fgrad ? 1 : 0;
+  c.chunk = f.chunk;
   const bool va = aligned16(p.V) && p.v_bs % 4 == 0;
   if (fgrad) c.v_mode = va && p.g.SC % 4 == 0 ? CT_RVEC : CT_RSCL;
   else if (p.v_trans) c.v_mode = va && p.v_ld % 4 == 0 ? CT_RVEC : CT_RSCL;

@@ -39,9 +39,9 @@ cudaError_t code_launch_s(cudaStream_t st, const CodeParams& cp, int shape, int 
 }  // namespace
 
 CodeTile code_tile(int shape) {
-  if (shape == 0) return {CT_ROWS, 256, (size_t)CodeAcc<64, 256>::SLOT_FLOATS * 8};
-  if (shape == 1) return {CT_ROWS, 128, (size_t)CodeAcc<64, 128>::SLOT_FLOATS * 8};
-  return {CT_ROWS, 64, (size_t)CodeAcc<64, 64>::SLOT_FLOATS * 8};
+  if (shape == 0) return {CT_ROWS, 256, (size_t)CodeAcc<64, 256>::SLOT_FLOATS * 8, CodeSmem<64, 256>::NACC};
+  if (shape == 1) return {CT_ROWS, 128, (size_t)CodeAcc<64, 128>::SLOT_FLOATS * 8, CodeSmem<64, 128>::NACC};
+  return {CT_ROWS, 64, (size_t)CodeAcc<64, 64>::SLOT_FLOATS * 8, CodeSmem<64, 64>::NACC};
 }
 
 cudaError_t code_gemm_launch(cudaStream_t st, const CodeParams& cp, int shape, int device) {

@@ -13,12 +13,13 @@
 // forms sum_s F * G exactly (small integers times one power of two), so the product of every
 // element pair is the table's, and adds it to an FP32 accumulator in tensor memory.
 //
-// The accumulator add truncates (measured: one round toward zero per instruction, with at least 34
-// fraction bits kept before it), where an FP32 add rounds to nearest.  So every 128 reduction steps
-// the tile is added (round to nearest) to an FP32 partial tile in scratch and the tensor-memory tile
-// starts from zero: truncation errors never add up over more than 128 steps.  Measured against the
-// reference-order result the path is within 4e-8 (short reductions) to 3e-7 (10^5 steps), like the
-// split sums of the shared-memory kernels.
+// The accumulator add truncates (measured: one round toward zero per instruction, with at least 34 fraction bits kept
+// before it), where an FP32 add rounds to nearest; a 128-slot product is two instructions.  So after a chunk of the
+// reduction the tile is added (round to nearest) to an FP32 partial tile in scratch and tensor memory starts from zero;
+// tiles of 128 and 64 columns spread a chunk over two and three accumulators.  A chunk is as long as leaves the error
+// against 64 bits no larger than the table kernels' (code_steps in amsim.cu): with ordinary activations, weights and
+// gradients 3e-9 (64 steps) to 1e-7 (10^5 steps) on either path.  Operands whose exponents spread widely lose more here:
+// normal variates times 2^-10 .. 2^10 give 2e-6 (128 slots: 3.4e-6) where the table kernels give 1e-7 to 5e-7.
 //
 // Two CTAs (one pair of multiprocessors) share a tile of 256 rows and up to 256 columns (tcgen05 cta_group::2): each
 // encodes 128 rows of V and half the columns of U, the tensor cores read both halves, and the CTA of rank 0 issues.
@@ -49,7 +50,6 @@ constexpr int CT_KB = 16;        // reduction steps per block; a warp fetches an
 constexpr int CT_HALF = CT_KB / 2;
 constexpr int CT_RAW = 32 * CT_HALF * 4;  // one cp.async buffer of a warp
 constexpr int CT_ROWS = 256;     // rows of a CTA pair's tile
-constexpr int CT_CHUNK = 8;      // blocks summed in tensor memory before they go to the FP32 partial tile
 constexpr int CT_MAXSPIN = 1 << 20;  // bound on every wait (a wait gives up, the kernel drains and reports)
 
 // How an operand's elements sit in memory.
@@ -68,6 +68,7 @@ struct CodeParams {
   int v_mode, u_mode;        // CT_* of the operands
   int step_v, step_u;        // blocks never straddle a tap and offsets fit 32 bits: step through them
   int fgrad;                 // V is gathered along p with the reduction over grid positions
+  int chunk;                 // blocks summed in tensor memory before they go to the FP32 partial tile
   unsigned* stuck;           // set when a bounded wait ran out
 };
 
@@ -87,13 +88,15 @@ struct CodeSmem {
   static constexpr int NW = 2 * (4 + GU);         // two warps per group of 32 rows or columns
   static constexpr int NT = 32 * (NW + 1);
   static constexpr int NBH = (BN + 127) / 128;    // 512-byte scale chunks of U per word (both halves: every CTA needs all)
-  static constexpr int NST = BN == 256 ? 6 : 8;   // stages in flight: tensor memory and shared memory hold no more
+  static constexpr int NST = BN == 64 ? 8 : 6;    // stages in flight: tensor memory and shared memory hold no more
+  // accumulators that a chunk's stages take in turn, added when the chunk is taken out: each has a NACC-th of the steps
+  static constexpr int NACC = BN == 64 ? 3 : BN == 128 ? 2 : 1;
   static constexpr int CODE_BYTES = BN / 2 * 128; // the codes of V go to tensor memory
   static constexpr int SF_BYTES = (1 + NBH) * C::W * 512;
   static constexpr int OFF_SF = NST * CODE_BYTES;
   static constexpr int OFF_RAW = OFF_SF + NST * SF_BYTES;
   // tensor memory columns: accumulators, NST stages of V codes, two sets of scales
-  static constexpr int T_CODES = BN;
+  static constexpr int T_CODES = NACC * BN;
   static constexpr int T_SF = T_CODES + NST * 32;
   static constexpr int SF_COLS = (1 + NBH) * C::W * 4;
   static_assert(T_SF + 2 * SF_COLS <= 512, "tensor memory");
@@ -710,10 +713,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
       decode_tile(run_at, tp, tq, tz, kb0, kb1);
       run_at += kb1 - kb0;
       const uint32_t idesc = code_idesc(tile_columns(tq));
-      for (int kb = kb0; kb < kb1; kb += CT_CHUNK, ++chunk) {
-        const int stages = (min(kb1, kb + CT_CHUNK) - kb) * C::STAGES_PER_KB;
+      for (int kb = kb0; kb < kb1; kb += cp.chunk, ++chunk) {
+        const int stages = (min(kb1, kb + cp.chunk) - kb) * C::STAGES_PER_KB;
         wt.wait_warp(bar_free, (chunk & 1) ^ 1);
-        uint32_t accumulate = 0;
+        uint32_t acc = 0;  // first column of the stage's accumulator
 #pragma unroll 1
         for (int i = 0; i < stages; ++i) {
           wt.wait(bar_full + 8 * b, phase);
@@ -733,15 +736,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
 #pragma unroll
             for (int s = 0; s < 4; ++s) {  // 64 code steps each; their two scale bytes sit in half (id 0 / 2) of a word
               const int word = S == 128 ? 0 : s >> 1, id = S == 128 ? (s >> 1) * 2 : (s & 1) * 2;
-              mma_codes(tmem, at + 8 * s, bd + 2 * s, idesc | ((uint32_t)id << 4) | ((uint32_t)id << 29), sf_t + word * 4,
-                        sfu_t + word * L::NBH * 4, s > 0 ? 1u : accumulate);
+              mma_codes(tmem + acc, at + 8 * s, bd + 2 * s, idesc | ((uint32_t)id << 4) | ((uint32_t)id << 29), sf_t + word * 4,
+                        sfu_t + word * L::NBH * 4, s > 0 || i >= L::NACC);
             }
             tc_commit(bar_empty + 8 * b);
             if (i + 1 == stages) tc_commit(bar_done);
           }
           __syncwarp();
-          accumulate = 1;
           sfset ^= 1;
+          acc = acc + BN == L::NACC * BN ? 0 : acc + BN;
           if (++b == NST) {
             b = 0;
             phase ^= 1;
@@ -832,7 +835,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
     // Takes this thread's units of a finished chunk out of tensor memory, adds what earlier chunks of the segment
     // left in the slot (first: nothing) and hands them on; the next chunk's products may begin once all are out.
     // The tensor core idles meanwhile, so the slot is read a unit ahead, from before the chunk is done.
-    auto take_chunk = [&](bool first, auto&& use) {
+    auto take_chunk = [&](bool first, int stages, auto&& use) {
       const int units = (A::UNITS - grp + NG - 1) / NG;
       float s[16];
       if (!first) read_slot(0, s);
@@ -841,7 +844,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
 #pragma unroll 1
       for (int i = 0; i < units; ++i) {
         float v[16];
-        tmem_load16(tmem + ((uint32_t)(w & 3) << 21) + (grp + i * NG) * 16, v);
+        const uint32_t at = tmem + ((uint32_t)(w & 3) << 21) + (grp + i * NG) * 16;
+        tmem_load16(at, v);
+#pragma unroll
+        for (int a = 1; a < L::NACC; ++a) {
+          if (a >= stages) break;  // (a chunk of fewer stages than accumulators)
+          float more[16];
+          tmem_load16(at + a * BN, more);
+#pragma unroll
+          for (int c = 0; c < 16; ++c) v[c] = __fadd_rn(v[c], more[c]);
+        }
         if (i + 1 == units) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
@@ -857,7 +869,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
     };
     // Moves a finished chunk of the segment to the slot.
     auto drain = [&](bool first) {
-      if (grp < NG) take_chunk(first, park_unit);
+      if (grp < NG) take_chunk(first, cp.chunk * C::STAGES_PER_KB, park_unit);
       ++chunk;
     };
 
@@ -876,20 +888,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
       }
       slot = prm.ws + (((long long)pair * 2 + (kb0 == 0 ? 1 : 0)) * 2 + rank) * A::SLOT_FLOATS + t;
       bool pending = false, fresh = true;
-      int ahead = half * SPH;  // own stages of the next chunk start here
+      int kc = kb0;  // first block of the chunk
       for (int kb = kb0; kb < kb1; ++kb) {
         fetch_next();
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
         const uint32_t rb = raw_s + buf * CT_RAW;
         buf ^= 1;
-        // the next chunk's first stages are made while the last one finishes, as many as the ring holds: a finished
-        // chunk is taken out at once (until then the tensor core idles)
-        if (pending && (ahead + SPH > NST || __all_sync(0xffffffffu, mbar_test(bar_done, chunk & 1)))) {
+        // the next chunk's first stages are made while the last one finishes, as many as the ring holds and at most one
+        // chunk: a finished chunk is taken out at once (until then the tensor core idles)
+        if (pending && ((kb - kc) * C::STAGES_PER_KB + half * SPH + SPH > NST || kb - kc == cp.chunk - 1 ||
+                        __all_sync(0xffffffffu, mbar_test(bar_done, chunk & 1)))) {
           drain(fresh);
           fresh = pending = false;
         }
-        ahead += C::STAGES_PER_KB;
 #pragma unroll
         for (int j = 0; j < SPH; ++j) {
           uint32_t x[KS];
@@ -973,9 +985,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
           advance(1);
         }
         advance(SPH);
-        if ((kb - kb0 + 1) % CT_CHUNK == 0 && kb + 1 < kb1) {
-          pending = true;
-          ahead = half * SPH;
+        if (kb - kc == cp.chunk - 1) {
+          kc = kb + 1;
+          pending = kc < kb1;
         }
       }
       if (pending) {
@@ -1008,7 +1020,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
           }
           if (!finite) odd_s = 1;
         };
-        take_chunk(fresh, [&](int i, const float (&v)[16]) {
+        take_chunk(fresh, ((kb1 - kb0 - 1) % cp.chunk + 1) * C::STAGES_PER_KB, [&](int i, const float (&v)[16]) {
           if (shared_tile) park_unit(i, v);
           else write_unit(i, v);
         });
@@ -1042,7 +1054,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
               float v[16];
 #pragma unroll
               for (int c = 0; c < 16; ++c) v[c] = 0.f;
-              // the sharers' tiles four at a time: 16 loads in flight (one tile after the other took a round trip to L2 each)
+              // The sharers' tiles four at a time: 16 loads in flight (one tile after the other took a round trip to L2 each).
+              // Four are summed before they are added: 74 tiles added one by one rounded the whole sum 74 times (filter
+              // gradient of 64 x 256 over 96800 pixels: 1.58e-7 from the exact sum, fours 9.7e-8, the table kernels 9.8e-8).
               for (int run = c0; run <= c1; run += 4) {
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
@@ -1057,11 +1071,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
                       part[r][c] = run + r <= c1 && AMSIM_IN(prm, BUF_WS, at, float) ? __ldcg(at) : 0.f;
                     }
                   }
+                  // (in this order: sums of pairs took 150 bytes more of spills and 10 % more of 3x3 256 -> 256's time)
 #pragma unroll
-                  for (int r = 0; r < 4; ++r)
-                    if (run + r <= c1)
+                  for (int r = 2; r >= 0; --r)
 #pragma unroll
-                      for (int c = 0; c < 4; ++c) v[h * 4 + c] = __fadd_rn(v[h * 4 + c], part[r][c]);
+                    for (int c = 0; c < 4; ++c) part[r][c] = __fadd_rn(part[r][c], part[r + 1][c]);
+#pragma unroll
+                  for (int c = 0; c < 4; ++c) v[h * 4 + c] = __fadd_rn(v[h * 4 + c], part[0][c]);
                 }
               }
               write_unit(i, v);

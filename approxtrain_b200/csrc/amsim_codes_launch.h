@@ -11,6 +11,7 @@ struct CodeParams;
 struct CodeTile {
   int bm, bn;
   size_t slot_bytes;  // one parked tile (both CTAs' halves)
+  int accumulators;   // tiles in tensor memory whose sum is a chunk's
 };
 CodeTile code_tile(int shape);
 cudaError_t code_gemm_launch(cudaStream_t st, const CodeParams& cp, int shape, int device);

@@ -2,9 +2,11 @@
 deterministic mode, which is bit-identical to the reference: every table factorisation (32, 64 and 128
 slots), every operand layout the kernel fetches, and the sizes where its tiles and stages end.
 
-Bound: products are exact; a partial sum of at most 128 steps is truncated once per step, so it is off
-by at most 128 * 2^-23 of the partial sums' largest value (1.5e-5, if every step lost a whole bit), and
-about 2^-24 * sqrt(steps) on data whose products spread over many exponents: 1e-5 as for every fast kernel."""
+Bound: products are exact; an accumulator takes at most 128 steps (256 instructions with 128 slots) and each
+truncates by less than 2^-23 of a partial sum, half of that on average: at most 256 * 2^-24 = 1.5e-5 of the largest
+partial sum if every instruction lost bits.  A product has at most 9 significant bits, so with ordinary operands few
+do; with widely spread exponents nearly all do, on sums that grow over the chunk (the factor 1/2 of a mean):
+1e-5 as for every fast kernel.  test_no_further_from_64_bits compares both paths with exact sums."""
 import ctypes as C
 import os
 
@@ -100,9 +102,12 @@ def test_products_up_to_the_largest_float(forced, lut, e):
     w[3, 3:90], x[5:40, 3] = -big, 2.0 ** (e - e // 2)      # the sum returns to ordinary size
     f = lambda: ops.denseam(x, w, lut_path(lut))  # noqa: E731
     got, want = _on(forced, 1, f), _on(forced, 0, f)
-    assert torch.isfinite(want).all()
-    assert torch.equal(got[5:40, 3:90], want[5:40, 3:90]) or rel_l2(got[5:40, 3:90].cpu().numpy(), want[5:40, 3:90].cpu().numpy()) <= 1e-5
-    assert torch.isfinite(got).all()
+    assert torch.isfinite(want).all() and torch.isfinite(got).all()
+    # 130 additions in any order, each off by at most 2^-23 of a partial sum of about 2^e
+    assert (got[5:40, 3:90].double() - want[5:40, 3:90]).abs().max() <= 130 * 2.0 ** (e - 22)
+    other = torch.ones_like(got, dtype=torch.bool)
+    other[5:40, 3:90] = False
+    _close(got[other], want[other])
 
 
 @pytest.mark.parametrize("lut", ["MBM_7", "MIT_7"])
@@ -140,6 +145,53 @@ def test_a_non_finite_operand_makes_its_outputs_nan_and_no_others(forced, lut):
     bad = torch.zeros(700, 200, dtype=torch.bool, device="cuda")
     bad[3], bad[600], bad[:, 11], bad[:, 190] = True, True, True, True
     assert torch.equal(torch.isnan(y), bad) and torch.equal(y[~bad], clean[~bad])
+
+
+def _exact_gemm(a, b, lut):
+    """sum_k AM(a[i, k], b[k, j]) in 64 bits, products from the elementwise op."""
+    from approxtrain_b200 import ops
+    m = int(lut.split("_")[1])
+    s = 1 + torch.arange(1 << m, device="cuda") / float(1 << m)
+    table = ops.am_multiply(s[:, None].expand(1 << m, 1 << m).contiguous(), s[None, :].expand(1 << m, 1 << m).contiguous(),
+                            lut_path(lut)).double().flatten()
+
+    def split(x):
+        bits = x.contiguous().view(torch.int32)
+        e = (bits >> 23) & 255
+        scale = torch.ldexp(torch.where(bits < 0, -1.0, 1.0).double(), (e - 127).double())
+        return torch.where(e > 0, scale, torch.zeros_like(scale)), ((bits >> (23 - m)) & ((1 << m) - 1)).long()
+    (sa, ia), (sb, ib) = split(a), split(b)
+    out = torch.zeros(a.shape[0], b.shape[1], dtype=torch.float64, device="cuda")
+    for k in range(a.shape[1]):
+        out += table[ia[:, k, None] * (1 << m) + ib[None, k]] * (sa[:, k, None] * sb[None, k])
+    return out
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7", "MIT_5"])
+@pytest.mark.parametrize("data", ["activations", "normal", "positive", "spread"])
+@pytest.mark.parametrize("k,q", [(64, 256), (147, 64), (256, 256), (512, 300), (576, 64), (1152, 128), (2304, 256)])
+def test_no_further_from_64_bits(forced, lut, data, k, q):
+    from approxtrain_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(k)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, w = r(512, k), r(k, q)
+    if data == "activations":
+        x, w = torch.relu(x), w * (2.0 / k) ** 0.5
+    elif data == "positive":
+        x, w = torch.rand(512, k, generator=g, device="cuda"), torch.rand(k, q, generator=g, device="cuda")
+    elif data == "spread":
+        x, w = (t * 2.0 ** torch.randint(-10, 11, t.shape, generator=g, device="cuda") for t in (x, w))
+    want = _exact_gemm(x, w, lut)
+    err = lambda y: float((y.double() - want).norm() / want.norm())  # noqa: E731
+    here, table = err(_on(forced, 1, lambda: ops.denseam(x, w, lut_path(lut)))), err(_on(forced, 0, lambda: ops.denseam(x, w, lut_path(lut))))
+    if data == "spread":
+        assert here <= 1e-5 / 2      # nearly every instruction truncates: half of 256 * 2^-24, on half the final sum
+    elif k < (64 if lut == "MBM_7" else 128):
+        pass                         # such reductions take this path only when it is forced
+    else:
+        # as close as the table kernels; few of the outputs are off at all in short reductions, so the two figures
+        # scatter by a tenth from seed to seed
+        assert here <= 1.2 * table, (here, table)
 
 
 def test_zeros_give_zero_and_non_finite_values_stay_visible(forced):
