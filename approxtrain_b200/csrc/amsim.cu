@@ -939,9 +939,9 @@ FgradPlan plan_fgrad(int P, int Q, int K, bool exact, int np, int sms) {
   return f;
 }
 
-// Workspace that covers whichever plan the launch takes (the wide kernel needs operands the
+// Workspace that covers whichever plan of the table kernels the launch takes (the wide kernel needs operands the
 // query cannot see: 16-byte aligned tensors, a table in shared memory).
-size_t fgrad_workspace(int P, int Q, int K, bool exact, int sms) {
+size_t fgrad_table_workspace(int P, int Q, int K, bool exact, int sms) {
   size_t need = plan_fgrad(P, Q, K, exact, 0, sms).ws_bytes;
   if (!exact) {
     for (int additive = 0; additive < 2; ++additive) {
@@ -950,10 +950,16 @@ size_t fgrad_workspace(int P, int Q, int K, bool exact, int sms) {
         if (np) need = std::max(need, plan_fgrad(P, Q, K, false, np, sms).ws_bytes);
       }
     }
-    const CodePlan c = plan_codes(P, Q, K, 1, sms, kCodeTraitsAny);
-    if (c.use) need = std::max(need, c.counter_bytes + c.slot_bytes);
   }
   return need;
+}
+// ... and of the tensor-core path; 0 where no table takes it.
+size_t fgrad_code_workspace(int P, int Q, int K, bool exact, int sms) {
+  const CodePlan c = plan_codes(P, Q, K, 1, sms, kCodeTraitsAny);
+  return !exact && c.use ? c.counter_bytes + c.slot_bytes : 0;
+}
+size_t fgrad_workspace(int P, int Q, int K, bool exact, int sms) {
+  return std::max(fgrad_table_workspace(P, Q, K, exact, sms), fgrad_code_workspace(P, Q, K, exact, sms));
 }
 
 template <int LM, int NP>
@@ -1508,24 +1514,24 @@ static void setup_wgrad(Params& p, const amsim_lut* lut, const float* x, const f
   fill_lut(p, lut, /*v_is_first_operand=*/!swap);
 }
 
-// Split-K scratch of a filter gradient; 0 for shapes the op itself refuses (check_conv_dims).
-static size_t conv_fgrad_workspace(int batch, int in_h, int in_w, int in_c, int f_h, int f_w, int out_c, int out_h,
-                                   int out_w, bool det, int sms) {
+// Scratch of a filter gradient, `plan` one of the fgrad_*_workspace; 0 for shapes the op itself refuses (check_conv_dims).
+static size_t conv_fgrad_workspace(size_t (*plan)(int, int, int, bool, int), int batch, int in_h, int in_w, int in_c, int f_h,
+                                   int f_w, int out_c, int out_h, int out_w, bool det, int sms) {
   if (batch <= 0 || in_c <= 0 || f_h <= 0 || f_w <= 0 || out_c <= 0 || out_h <= 0 || out_w <= 0) return 0;
   if (!prod3_below(f_h, f_w, in_c > out_c ? in_c : out_c, 1ll << 30) || !prod3_below(batch, out_h, out_w, (1ll << 31) - 256))
     return 0;
   const long long rows = (long long)f_h * f_w * in_c, npix = (long long)batch * out_h * out_w;
-  size_t need = fgrad_workspace((int)rows, out_c, (int)npix, det, sms);
+  size_t need = plan((int)rows, out_c, (int)npix, det, sms);
   // a 1x1 stride-1 convolution may run with the operand roles swapped (wgrad_swap): cover both plans
   if (f_h == 1 && f_w == 1 && out_h == in_h && out_w == in_w && wgrad_swap(in_c, out_c))
-    need = std::max(need, fgrad_workspace(out_c, in_c, (int)npix, det, sms));
+    need = std::max(need, plan(out_c, in_c, (int)npix, det, sms));
   return need;
 }
 
 size_t amsim_conv2d_bwd_filter_workspace(int batch, int in_h, int in_w, int in_c, int f_h, int f_w, int out_c,
                                          int out_h, int out_w, unsigned flags) {
   if (flags & AMSIM_INT32) return 0;
-  return conv_fgrad_workspace(batch, in_h, in_w, in_c, f_h, f_w, out_c, out_h, out_w, flags & AMSIM_DETERMINISTIC,
+  return conv_fgrad_workspace(fgrad_workspace, batch, in_h, in_w, in_c, f_h, f_w, out_c, out_h, out_w, flags & AMSIM_DETERMINISTIC,
                               sm_count(current_device()));
 }
 
@@ -1598,20 +1604,23 @@ int amsim_conv2d_bwd_filter_static(void* stream, const amsim_lut* lut, const flo
   if (rc) return rc;
   rc = check_conv_dims(batch, in_h, in_w, in_c, f_h, f_w, out_c, out_h, out_w, stride_h, stride_w, pad_top, pad_left);
   if (rc) return rc;
-  // the plan the launch will take: direct models always run unsplit (ordered chains), as in launch_fgrad
+  // What has to fit is a plan of the table kernels (direct models always run unsplit, as in launch_fgrad); launch_fgrad takes
+  // the tensor-core path only where that fits too.
   const bool det = (flags & AMSIM_DETERMINISTIC) || lut->direct;
-  const size_t need = (flags & AMSIM_INT32) ? 0
-                                            : conv_fgrad_workspace(batch, in_h, in_w, in_c, f_h, f_w, out_c, out_h, out_w,
-                                                                   det, sm_count(lut->device));
+  const int sms = sm_count(lut->device);
+  auto scratch_of = [&](size_t (*plan)(int, int, int, bool, int)) -> size_t {
+    return (flags & AMSIM_INT32) ? 0 : conv_fgrad_workspace(plan, batch, in_h, in_w, in_c, f_h, f_w, out_c, out_h, out_w, det, sms);
+  };
+  const size_t need = scratch_of(fgrad_table_workspace);
   if (need > (size_t)AMSIM_STATIC_SCRATCH_BYTES)
     return fail(AMSIM_ERR_WORKSPACE,
                 "this shape needs %zu bytes of split-K scratch, the built-in buffer holds %u: "
                 "use amsim_conv2d_bwd_filter with a caller-provided workspace",
                 need, (unsigned)AMSIM_STATIC_SCRATCH_BYTES);
   void* scratch = nullptr;
-  if (need > 0 && (rc = static_scratch_address(lut->device, &scratch))) return rc;
+  if ((need > 0 || scratch_of(fgrad_code_workspace) > 0) && (rc = static_scratch_address(lut->device, &scratch))) return rc;
   return amsim_conv2d_bwd_filter(stream, lut, x, dy, dw, batch, in_h, in_w, in_c, f_h, f_w, out_c, out_h, out_w,
-                                 stride_h, stride_w, pad_top, pad_left, scratch, need, flags);
+                                 stride_h, stride_w, pad_top, pad_left, scratch, scratch ? AMSIM_STATIC_SCRATCH_BYTES : 0, flags);
 }
 
 // ---- bias gradient ------------------------------------------------------------------------------

@@ -201,7 +201,7 @@ int amsim_conv2d_bwd_filter(void* stream, const amsim_lut* lut, const float* x,
  * TensorFlow allocator.)
  *
  * Same computation, same split plan and therefore bit-identical results as
- * amsim_conv2d_bwd_filter, but the split-K partial sums live in a buffer that
+ * amsim_conv2d_bwd_filter (one exception below), but the split-K partial sums live in a buffer that
  * is part of the library image on the device (AMSIM_STATIC_SCRATCH_BYTES,
  * resident on every GPU that loads the library until the process exits)
  * instead of a caller-supplied workspace.  It is meant for hosts that have no
@@ -211,8 +211,11 @@ int amsim_conv2d_bwd_filter(void* stream, const amsim_lut* lut, const float* x,
  * synchronises the whole device.  The call itself performs no cudaMalloc /
  * cudaFree and calls nothing that allocates device memory.
  *
- *  - A shape whose plan needs more than AMSIM_STATIC_SCRATCH_BYTES is refused
+ *  - A shape whose split plan needs more than AMSIM_STATIC_SCRATCH_BYTES is refused
  *    with AMSIM_ERR_WORKSPACE (nothing is launched); use the workspace variant.
+ *  - AMSIM_FAST only: where the workspace variant runs on the tensor cores with more
+ *    scratch than that, this call runs the table kernels: the same products, summed in
+ *    the order that the workspace variant takes when it is handed no more than that.
  *  - The first call on a device looks up the buffer's device address
  *    (cudaGetSymbolAddress); make that first call before starting any stream
  *    capture on that device.
