@@ -680,9 +680,6 @@ struct CodeTraits {
   bool additive;       // the other path needs no lookups
   bool fgrad, scalar;  // a filter gradient; operands that are fetched element by element
 };
-// The traits for which the path is taken most readily: the *_workspace functions do not know the table.
-constexpr CodeTraits kCodeTraitsAny = {32, false, true, false};
-
 // 16-step blocks that one accumulator in tensor memory takes before its sum goes on in FP32.  Its adds truncate, which costs
 // in proportion to their number, where one FP32 chain's rounding grows with the square root of its length: the shorter the
 // reduction, the shorter the chunk.  Errors against 64 bits (normal operands; table kernels / 16 / 32 / 64 / 128 steps):
@@ -715,8 +712,8 @@ double table_us(double products, int K, const CodeTraits& t) {
   return wide + (t.fgrad ? 0 : std::min(45.0, (t.additive ? 0.019 : 0.022) * std::max(0, K - 512)));
 }
 
-// Whether and how the tensor-core path runs a P x Q x K problem.  The grid depends on the dimensions, the device and
-// the debug switches only, so that a workspace sized for kCodeTraitsAny fits every launch.
+// Whether and how the tensor-core path runs a P x Q x K problem: depends on the dimensions, the table, the device and the
+// debug switches only, so a workspace sized for every table (fgrad_code_workspace) fits every launch.
 CodePlan plan_codes(int P, int Q, int K, int batch, int sms, const CodeTraits& t) {
   CodePlan f;
   // a switch that picks among the table kernels keeps the launch on them
@@ -955,8 +952,15 @@ size_t fgrad_table_workspace(int P, int Q, int K, bool exact, int sms) {
 }
 // ... and of the tensor-core path; 0 where no table takes it.
 size_t fgrad_code_workspace(int P, int Q, int K, bool exact, int sms) {
-  const CodePlan c = plan_codes(P, Q, K, 1, sms, kCodeTraitsAny);
-  return !exact && c.use ? c.counter_bytes + c.slot_bytes : 0;
+  size_t need = 0;
+  if (exact) return need;
+  for (const int slots : {32, 64, 128})
+    for (const bool additive : {false, true})
+      for (const bool scalar : {false, true}) {
+        const CodePlan c = plan_codes(P, Q, K, 1, sms, {slots, additive, true, scalar});
+        if (c.use) need = std::max(need, c.counter_bytes + c.slot_bytes);
+      }
+  return need;
 }
 size_t fgrad_workspace(int P, int Q, int K, bool exact, int sms) {
   return std::max(fgrad_table_workspace(P, Q, K, exact, sms), fgrad_code_workspace(P, Q, K, exact, sms));

@@ -205,6 +205,23 @@ def test_zeros_give_zero_and_non_finite_values_stay_visible(forced):
     assert not torch.isfinite(y[7]).any() and torch.equal(y[:7], torch.zeros(7, 96, device="cuda"))
 
 
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7", "MIT_5"])
+@pytest.mark.parametrize("rows,width,units", [(64, 4096, 4096), (100, 2048, 2050), (862, 925, 256), (900, 931, 250), (6272, 256, 1024)])
+def test_the_queried_workspace_serves_whatever_plan_is_taken(lut, rows, width, units):
+    """A launch that is handed more than the query asks for takes the same plan: the same bits."""
+    from approxtrain_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, dy = torch.randn(rows, width, generator=g, device="cuda"), torch.randn(rows, units, generator=g, device="cuda")
+    need = _lib.lib.amsim_dense_bwd_weight_workspace(rows, units, width, 0)
+
+    def grad(extra):
+        ws, dw = torch.empty(need + extra, dtype=torch.uint8, device="cuda"), torch.empty(width, units, device="cuda")
+        _lib.check(_lib.lib.amsim_dense_bwd_weight(ops._stream(), ops.get_lut(lut_path(lut), "cuda").handle, x.data_ptr(), dy.data_ptr(),
+                                                   dw.data_ptr(), rows, units, width, ws.data_ptr(), ws.numel(), 0))
+        return dw
+    assert torch.equal(grad(0), grad(128 << 20))
+
+
 def test_every_shipped_table_takes_the_path(forced):
     """With AMSIM_CODES=0 the table kernels run: another order of the same sum, so the bits differ."""
     from approxtrain_b200 import ops
