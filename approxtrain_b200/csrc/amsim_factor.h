@@ -43,6 +43,22 @@ struct Spare {
   std::vector<double> b;   // its G per column
 };
 
+// The constants a slot may have (bit c: kLevels[c]) for its G to be v divided by the constant.
+inline unsigned constants_of(double v) {
+  unsigned m = 0;
+  for (int c = 1; c < 8; ++c)
+    if (code_of(v / kLevels[c]) >= 0) m |= 1u << c;
+  return m;
+}
+// constants_of q quarters; only multiples of a quarter up to 36 have any.
+struct ConstantTable {
+  unsigned char of[145];
+  ConstantTable() {
+    for (int q = 0; q <= 144; ++q) of[q] = (unsigned char)constants_of(q / 4.0);
+  }
+  unsigned operator()(int q) const { return q <= 144 && q >= -144 ? of[q < 0 ? -q : q] : 0; }
+};
+
 // Splits rest[j] over at most n constant slots; false if it does not fit.
 inline bool split_rest(const std::vector<double>& rest, int n, std::vector<Spare>& out) {
   out.clear();
@@ -149,10 +165,25 @@ inline CodeTables factor_table(const uint8_t* entries, int m) {
       level.assign(nstep, 1);
       const std::vector<double> r0 = rest_of();
       std::vector<double> r(C);
-      for (int a = 0; a < nstep && !found; ++a)
+      // Most pairs leave a rest that no slot holds, and a column or two show it: quarters of the unit in integers, stopped
+      // there.  (With every column worked out in doubles first, a table of 128 x 128 without a factorisation took one to
+      // three seconds to open.)
+      const ConstantTable constants;
+      std::vector<int> q0(C);
+      std::vector<std::vector<int>> step4(nstep, std::vector<int>(C));
+      bool quarters = true;
+      for (int j = 0; j < C; ++j) {
+        quarters = quarters && std::fabs(r0[j]) < 1e6 && r0[j] * 4 == std::floor(r0[j] * 4);
+        q0[j] = quarters ? (int)(r0[j] * 4) : 0;
+        for (int s = 0; s < nstep; ++s) step4[s][j] = (int)(D[s][j] * 4);  // (codes: whole halves)
+      }
+      for (int a = 0; a < nstep && !found && quarters; ++a)
         for (int ca = -4; ca <= 3 && !found; ++ca)
           for (int b = a + 1; b < nstep && !found; ++b)
             for (int cb = -4; cb <= 3 && !found; ++cb) {
+              unsigned left = 0xFE;
+              for (int j = 0; j < C && left; ++j) left &= constants(q0[j] - (ca - 1) * step4[a][j] - (cb - 1) * step4[b][j]);
+              if (!left) continue;
               for (int j = 0; j < C; ++j) r[j] = r0[j] - (ca - 1) * D[a][j] - (cb - 1) * D[b][j];
               if (split_rest(r, spare > 1 ? 1 : spare, extra)) {
                 level[a] = ca;
