@@ -123,26 +123,26 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// bar: an address in the cluster's shared memory
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// Stores a word in the other CTA's shared memory and counts its four bytes there (both addresses the cluster's).
+// Stores a word in the other CTA's shared memory and counts its four bytes there (both addresses the cluster's).  The
+// count is a release in the scope of the cluster.  It also serves as the signal to the other CTA, with a word nobody reads:
+// an arrive that releases to the cluster waits for the thread's earlier accesses to reach it, and that made 3x3 64 -> 64 on
+// 32 x 55 x 55 take 1501 us instead of 1055 (forward and backward); an arrive without a scope releases to its own CTA only.
 __device__ __forceinline__ void st_async_remote(uint32_t addr, uint32_t v, uint32_t bar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// (every barrier here gets arrivals or counts from the other CTA too)
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+  asm volatile("{.reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {  // (does not wait)
   uint32_t ok;
-  asm volatile("{.reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+  asm volatile("{.reg .pred p; mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
@@ -628,6 +628,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
   __shared__ uint64_t bars[3 * NST + 2];
   __shared__ uint32_t tmem_holder;
   __shared__ int flag_s;
+  __shared__ uint32_t signal_s;  // where the other CTA's signals store their word
   __shared__ int odd_s;    // outputs that are not finite have been written (repair_outputs)
   __shared__ int wrote_s;  // this CTA has written its rows of the run's first (1) or last (2) tile, shared with other runs
   const Params& prm = cp.prm;
@@ -645,11 +646,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
   if (t == 0) {
     for (int i = 0; i < NST; ++i) {
       mbar_init(bar_full + 8 * i, NW / 2);  // half of the warps make a stage; the other CTA adds its scale bytes
-      mbar_init(bar_peer + 8 * i, 1);       // (rank 0) the other CTA's stage is full
+      mbar_init(bar_peer + 8 * i, 1);       // (rank 0) the other CTA's stage is full: its signal, and the issue warp expecting it
       mbar_init(bar_empty + 8 * i, 1);
     }
     mbar_init(bar_done, 1);
-    mbar_init(bar_free, 2 * 4 * NG);
+    mbar_init(bar_free, 4 * NG);            // (rank 0) this CTA's draining warps, and the other's signals
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     odd_s = wrote_s = 0;
   }
@@ -685,16 +686,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
 
   if (w == NW && rank != 0) {
     // ---- forwards "stage full" of this CTA to the issuing one: one warp fences for all, and the operand warps signal
-    // inside their CTA only (a proxy fence and a cluster-wide release in every one of them, with its own stores in
-    // flight, made 3x3 256 -> 256 on 64 x 14 x 14 take 483 us instead of 316)
-    const uint32_t lead = cluster_addr(bar_peer, 0);
+    // inside their CTA only.  The order: an operand warp's stores, its arrive (release in the CTA), this warp's wait, the
+    // fence to the proxy that the products read through, the signal (release in the cluster), the issue warp's wait.
+    const uint32_t lead = cluster_addr(bar_peer, 0), signal = cluster_addr(smem_addr(&signal_s), 0);
     uint32_t b = 0, phase = 0;
     const long long stages = (long long)(run_end - run_at) * C::STAGES_PER_KB;
     for (long long i = 0; i < stages; ++i) {
       wt.wait_warp(bar_full + 8 * b, phase);
       asm volatile("tcgen05.fence::after_thread_sync;\nfence.proxy.async.shared::cta;\ntcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive_remote(lead + 8 * b);
+      if (lane == 0) st_async_remote(signal, 0, lead + 8 * b);
       if (++b == NST) {
         b = 0;
         phase ^= 1;
@@ -719,6 +720,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
         uint32_t acc = 0;  // first column of the stage's accumulator
 #pragma unroll 1
         for (int i = 0; i < stages; ++i) {
+          if (lane == 0) mbar_arrive_expect(bar_peer + 8 * b, 4);
           wt.wait(bar_full + 8 * b, phase);
           wt.wait_warp(bar_peer + 8 * b, phase);
           asm volatile("tcgen05.fence::after_thread_sync;\nfence.proxy.async.shared::cta;" ::: "memory");
@@ -752,6 +754,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
         }
       }
     }
+    wt.wait_warp(bar_free, (chunk & 1) ^ 1);  // no signal is on its way to this CTA when it ends
   } else {
     // ---- operand warps: 32 rows of V (w < 8) or columns of U each, one half of every block ----------
     const bool is_v = w < 8;
@@ -777,7 +780,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
     const uint32_t code_t = tmem + L::T_CODES + ((uint32_t)(w & 3) << 21);
     uint32_t sf_off = L::OFF_SF + lane * 16 + group * 4;
     const uint32_t peer_smem = cluster_addr(smem0, rank ^ 1u), peer_full = cluster_addr(bar_full, rank ^ 1u);
-    const uint32_t lead_free = cluster_addr(bar_free, 0);
+    const uint32_t lead_free = cluster_addr(bar_free, 0), lead_signal = cluster_addr(smem_addr(&signal_s), 0);
 
     RowFetch rf;
     rf.k_at = half * CT_HALF;
@@ -857,7 +860,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
         if (i + 1 == units) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) mbar_arrive_remote(lead_free);
+          if (lane == 0) {
+            if (rank != 0) st_async_remote(lead_signal, 0, lead_free);
+            else if (w == 0) mbar_arrive_expect(bar_free, 4 * 4 * NG);
+            else mbar_arrive(bar_free);
+          }
         }
         if (!first) {
 #pragma unroll
