@@ -28,7 +28,7 @@ EXPORTS = [
     "amsim_dense_bwd_weight_workspace", "amsim_dense_bwd_weight", "amsim_dense_bwd_input", "amsim_matmul",
     "amsim_matmul_ex", "amsim_bias_grad_workspace", "amsim_bias_grad",
     "amsim_debug_fastdiv", "amsim_debug_launch_count", "amsim_debug_reload_env", "amsim_debug_bounds_report",
-    "amsim_debug_wait_report",
+    "amsim_async_status", "amsim_debug_wait_report",
 ]
 
 
@@ -79,6 +79,7 @@ def _load() -> C.CDLL:
     L.amsim_debug_launch_count.argtypes = []
     L.amsim_debug_launch_count.restype = C.c_ulonglong
     L.amsim_debug_bounds_report.argtypes = [C.POINTER(C.c_ulonglong)]
+    L.amsim_async_status.argtypes = []
     L.amsim_debug_wait_report.argtypes = [C.POINTER(C.c_uint)]
     L.amsim_debug_reload_env.argtypes = []
     L.amsim_debug_reload_env.restype = None

@@ -77,6 +77,7 @@ struct Switches {
   int capture_cluster = -1; // AMSIM_CAPTURE_CLUSTER=0/1 small launches inside a graph capture: balanced / cluster split
   int balanced_waves = -1;  // AMSIM_BALANCED_WAVES=n    CTAs of a balanced launch: n times the resident slots
   int codes = -1;           // AMSIM_CODES=0/1           tensor-core path of factorable tables: never / whenever eligible
+  int codes_spin = -1;      // AMSIM_CODES_SPIN=n        tries of a wait in that path's kernels (0: the first wait gives up)
   int bounds_shrink = 0;    // AMSIM_BOUNDS_SHRINK=n     bounds-checking build only: the output's recorded extent is n bytes
                             //                           short, so its last stores are caught (self-test of the checker)
 };
@@ -105,6 +106,7 @@ void load_switches() {
   tri("AMSIM_CAPTURE_CLUSTER", w.capture_cluster);
   tri("AMSIM_BALANCED_WAVES", w.balanced_waves);
   tri("AMSIM_CODES", w.codes);
+  tri("AMSIM_CODES_SPIN", w.codes_spin);
   tri("AMSIM_BOUNDS_SHRINK", w.bounds_shrink);
   g_sw = w;
 }
@@ -197,6 +199,32 @@ namespace {
 std::mutex g_lut_mu;
 std::map<std::string, amsim_lut*> g_lut_cache;
 
+// Words in host memory, one per device, that a tensor-core kernel sets when a bounded wait of its warps has run out (its
+// results are wrong).  Allocated with the first table that has such kernels; read, without synchronising, by every call.
+constexpr int kMostDevices = 64;
+std::atomic<unsigned*> g_stuck{nullptr};
+
+int stuck_words_open() {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  if (g_stuck.load()) return AMSIM_OK;
+  void* p = nullptr;
+  CUDA_TRY(cudaHostAlloc(&p, kMostDevices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped));
+  memset(p, 0, kMostDevices * sizeof(unsigned));
+  g_stuck.store(static_cast<unsigned*>(p));
+  return AMSIM_OK;
+}
+// Whether a wait has run out on the device since the last time this was asked.
+bool take_stuck(int device) {
+  unsigned* const words = g_stuck.load(std::memory_order_acquire);
+  if (!words || device < 0 || device >= kMostDevices) return false;
+  return *(volatile unsigned*)(words + device) != 0 && __atomic_exchange_n(words + device, 0u, __ATOMIC_RELAXED) != 0;
+}
+int report_stuck(int device) {
+  if (!take_stuck(device)) return AMSIM_OK;
+  return fail(AMSIM_ERR_CUDA, "a tensor-core kernel of an earlier call gave up waiting between its warps: the results of that call are wrong");
+}
+
 // approx_mul_lut.h:22-25
 int parse_mant_width(const char* path) {
   const char* us = strrchr(path, '_');
@@ -285,8 +313,9 @@ int upload_lut(const uint8_t* bytes, int m, int device, amsim_lut** out) {
     if (e == cudaSuccess) e = cudaMemcpy(h->d_trans, trans.data(), h->enc_bytes, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) bail(e, "upload of encoded lut");
     if (rc == AMSIM_OK) {
-      h->codes = amsim::factor_table(canon.data(), m);
-      if (h->codes.slots) {
+      if (device < kMostDevices) h->codes = amsim::factor_table(canon.data(), m);
+      if (h->codes.slots) rc = stuck_words_open();
+      if (rc == AMSIM_OK && h->codes.slots) {
         e = cudaMalloc(&h->d_codes_f, h->codes.f.size());
         if (e == cudaSuccess) e = cudaMalloc(&h->d_codes_g, h->codes.g.size());
         if (e == cudaSuccess) e = cudaMemcpy(h->d_codes_f, h->codes.f.data(), h->codes.f.size(), cudaMemcpyHostToDevice);
@@ -329,7 +358,7 @@ int check_common(const amsim_lut* lut, unsigned flags, bool need_gemm) {
   CUDA_TRY(cudaGetDevice(&dev));
   if (dev != lut->device)
     return fail(AMSIM_ERR_INVALID, "current device %d differs from the LUT's device %d", dev, lut->device);
-  return AMSIM_OK;
+  return report_stuck(dev);
 }
 
 template <typename K>
@@ -649,23 +678,6 @@ int launch_gather_t(cudaStream_t st, Params& p, int batch, int device) {
 }
 
 // ---- tensor-core path of factorable tables (amsim_codes.cuh) ------------------------------------
-// Set by a kernel whose bounded wait ran out (its results are wrong); read by amsim_debug_wait_report.
-__device__ unsigned g_code_stuck;
-
-int code_stuck_address(int device, unsigned** out) {
-  static std::mutex mu;
-  static std::map<int, unsigned*> known;
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = known.find(device);
-  if (it == known.end()) {
-    void* p = nullptr;
-    CUDA_TRY(cudaGetSymbolAddress(&p, g_code_stuck));
-    it = known.emplace(device, static_cast<unsigned*>(p)).first;
-  }
-  *out = it->second;
-  return AMSIM_OK;
-}
-
 struct CodePlan {
   int use = 0, shape = 0, chunk = 1;
   long long tiles = 0, iters = 0;
@@ -761,6 +773,7 @@ void code_params(CodeParams& c, const Params& p, const CodePlan& f, bool fgrad) 
   c.sh_u = p.ct_sh_u;
   c.unit = p.ct_unit;
   c.fgrad = fgrad ? 1 : 0;
+  c.spins = sw().codes_spin >= 0 ? sw().codes_spin : CT_MAXSPIN;
   c.chunk = f.chunk;
   const bool va = aligned16(p.V) && p.v_bs % 4 == 0;
   if (fgrad) c.v_mode = va && p.g.SC % 4 == 0 ? CT_RVEC : CT_RSCL;
@@ -782,8 +795,7 @@ int launch_codes(cudaStream_t st, const Params& p, const CodePlan& f, bool fgrad
   code_params(c, p, f, fgrad);
   c.prm.ws = static_cast<float*>(parked);
   c.prm.sk_count = static_cast<int*>(counters);
-  int rc = code_stuck_address(device, &c.stuck);
-  if (rc) return rc;
+  c.stuck = g_stuck.load() + device;
   AMSIM_COUNT_LAUNCH();
   CUDA_TRY(code_gemm_launch(st, c, f.shape, device));
   return AMSIM_OK;
@@ -1198,14 +1210,12 @@ int amsim_debug_bounds_report(unsigned long long* word) {
 int amsim_debug_wait_report(unsigned* stuck) {
   if (!stuck) return fail(AMSIM_ERR_INVALID, "NULL argument");
   *stuck = 0;
-  unsigned* p = nullptr;
-  int rc = code_stuck_address(current_device(), &p);
-  if (rc) return rc;
   CUDA_TRY(cudaDeviceSynchronize());
-  CUDA_TRY(cudaMemcpy(stuck, p, sizeof(*stuck), cudaMemcpyDeviceToHost));
-  CUDA_TRY(cudaMemset(p, 0, sizeof(*stuck)));
+  *stuck = take_stuck(current_device());
   return AMSIM_OK;
 }
+
+int amsim_async_status(void) { return report_stuck(current_device()); }
 
 void amsim_debug_reload_env(void) {
   sw();  // make sure the one-time load has happened, then replace its result

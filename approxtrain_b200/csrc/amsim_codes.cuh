@@ -50,7 +50,7 @@ constexpr int CT_KB = 16;        // reduction steps per block; a warp fetches an
 constexpr int CT_HALF = CT_KB / 2;
 constexpr int CT_RAW = 32 * CT_HALF * 4;  // one cp.async buffer of a warp
 constexpr int CT_ROWS = 256;     // rows of a CTA pair's tile
-constexpr int CT_MAXSPIN = 1 << 20;  // bound on every wait (a wait gives up, the kernel drains and reports)
+constexpr int CT_MAXSPIN = 1 << 20;  // bound on every wait (see Waiter)
 
 // How an operand's elements sit in memory.
 constexpr int CT_KVEC = 0;   // 16-byte groups of four consecutive reduction steps of one row
@@ -69,7 +69,8 @@ struct CodeParams {
   int step_v, step_u;        // blocks never straddle a tap and offsets fit 32 bits: step through them
   int fgrad;                 // V is gathered along p with the reduction over grid positions
   int chunk;                 // blocks summed in tensor memory before they go to the FP32 partial tile
-  unsigned* stuck;           // set when a bounded wait ran out
+  int spins;                 // bound on every wait
+  unsigned* stuck;           // (host memory) set when a bounded wait ran out
 };
 
 template <int S>
@@ -221,17 +222,19 @@ __device__ __forceinline__ void cp_async16n(uint32_t dst, const void* src, int b
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-// Waits for a phase of an mbarrier, at most CT_MAXSPIN tries; after a wait has run out every later
-// one of this thread passes at once, so the kernel runs to its end (with wrong results) and reports.
+// Waits for a phase of an mbarrier, at most `spins` tries.  A thread whose wait has run out is dead: it waits no more, signals
+// nobody and issues nothing, so the warps that depend on it run out too, and only walks its work to the end (the tile
+// counters stay in step, the results are wrong).  The host reads the mark at the next call.
 struct Waiter {
   unsigned* stuck;
+  int spins;
   bool dead;
   __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity) {
     if (dead) return;
-    for (int i = 0; i < CT_MAXSPIN; ++i)
+    for (int i = 0; i < spins; ++i)
       if (mbar_try(bar, parity)) return;
     dead = true;
-    atomicExch(stuck, 1u);
+    *(volatile unsigned*)stuck = 1u;
   }
   __device__ __forceinline__ void wait_warp(uint32_t bar, uint32_t parity) {
     wait(bar, parity);
@@ -625,7 +628,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
   constexpr int NW = L::NW, GU = L::GU, KS = C::KS, W = C::W, CH = C::CH, REP = C::REP, NST = L::NST;
   constexpr int NG = A::NG, UPT = A::UPT;
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  __shared__ uint64_t bars[3 * NST + 2];
+  __shared__ uint64_t bars[3 * NST + 3];
   __shared__ uint32_t tmem_holder;
   __shared__ int flag_s;
   __shared__ uint32_t signal_s;  // where the other CTA's signals store their word
@@ -641,7 +644,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
   const int pair = blockIdx.x >> 1;
   const uint32_t bar0 = smem_addr(bars);
   const uint32_t bar_full = bar0, bar_empty = bar0 + 8 * NST, bar_peer = bar0 + 16 * NST, bar_done = bar0 + 24 * NST,
-                 bar_free = bar_done + 8;
+                 bar_free = bar_done + 8, bar_exit = bar_done + 16;
 
   if (t == 0) {
     for (int i = 0; i < NST; ++i) {
@@ -650,6 +653,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
       mbar_init(bar_empty + 8 * i, 1);
     }
     mbar_init(bar_done, 1);
+    mbar_init(bar_exit, 1);
     mbar_init(bar_free, 4 * NG);            // (rank 0) this CTA's draining warps, and the other's signals
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     odd_s = wrote_s = 0;
@@ -682,7 +686,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
   };
   // columns of U in the products of tile column tq; each CTA encodes one half of them
   auto tile_columns = [&](int tq) { return min(BN, (prm.Q - tq * BN + 63) / 64 * 64); };
-  Waiter wt{cp.stuck, false};
+  Waiter wt{cp.stuck, cp.spins, false};
 
   if (w == NW && rank != 0) {
     // ---- forwards "stage full" of this CTA to the issuing one: one warp fences for all, and the operand warps signal
@@ -695,7 +699,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
       wt.wait_warp(bar_full + 8 * b, phase);
       asm volatile("tcgen05.fence::after_thread_sync;\nfence.proxy.async.shared::cta;\ntcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) st_async_remote(signal, 0, lead + 8 * b);
+      if (lane == 0 && !wt.dead) st_async_remote(signal, 0, lead + 8 * b);
       if (++b == NST) {
         b = 0;
         phase ^= 1;
@@ -720,7 +724,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
         uint32_t acc = 0;  // first column of the stage's accumulator
 #pragma unroll 1
         for (int i = 0; i < stages; ++i) {
-          if (lane == 0) mbar_arrive_expect(bar_peer + 8 * b, 4);
+          if (lane == 0 && !wt.dead) mbar_arrive_expect(bar_peer + 8 * b, 4);
           wt.wait(bar_full + 8 * b, phase);
           wt.wait_warp(bar_peer + 8 * b, phase);
           asm volatile("tcgen05.fence::after_thread_sync;\nfence.proxy.async.shared::cta;" ::: "memory");
@@ -728,7 +732,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
           const uint32_t at = tmem + L::T_CODES + b * 32;
           const uint32_t sf_t = tmem + L::T_SF + sfset * L::SF_COLS;  // scale columns: V [word], U [word][128 columns]
           const uint32_t sfu_t = sf_t + W * 4;
-          if (elected) {
+          if (elected && !wt.dead) {
 #pragma unroll
             for (int j = 0; j < W; ++j) scales_to_tmem(sf_t + 4 * j, sfd + 32 * j);
 #pragma unroll
@@ -860,7 +864,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
         if (i + 1 == units) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) {
+          if (lane == 0 && !wt.dead) {
             if (rank != 0) st_async_remote(lead_signal, 0, lead_free);
             else if (w == 0) mbar_arrive_expect(bar_free, 4 * 4 * NG);
             else mbar_arrive(bar_free);
@@ -981,11 +985,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
 #pragma unroll
             for (int i = 0; i < W; ++i) {
               sts32(smem0 + sf_at + 512 * i, sf[i]);
-              if (sends) st_async_remote(peer_smem + sf_at + 512 * i, sf[i], peer_full + 8 * b);  // both CTAs need every column's scales
+              if (sends && !wt.dead) st_async_remote(peer_smem + sf_at + 512 * i, sf[i], peer_full + 8 * b);  // both CTAs need every column's scales
             }
           }
           __syncwarp();
-          if (lane == 0) {
+          if (lane == 0 && !wt.dead) {
             if (is_v && group == 0) mbar_arrive_expect(bar_full + 8 * b, own * 4 * W);
             else mbar_arrive(bar_full + 8 * b);
           }
@@ -1095,6 +1099,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CodeSmem<S, BN>::NT,
       ++chunk;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  if (w == NW) {
+    // Products that a dead warp left in flight have to end before the tensor memory goes.  (Otherwise this passes at once.)
+    if (rank == 0 && elect_lane()) tc_commit(bar_exit);
+    Waiter last{cp.stuck, CT_MAXSPIN, false};
+    last.wait_warp(bar_exit, 0);
+    if (wt.dead) __nanosleep(100000);  // signals of other warps to this CTA
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

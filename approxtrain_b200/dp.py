@@ -23,6 +23,13 @@ import torch
 import torch.distributed as dist
 
 
+def _check_kernels() -> None:
+    """Raises if a captured kernel of an earlier replay gave up a wait (the library's calls check this
+    themselves; a replay makes none)."""
+    from ._lib import check, lib
+    check(lib.amsim_async_status())
+
+
 class DataParallelSGD:
     def __init__(self, model: torch.nn.Module, lr: float, bucket_bytes: int = 32 << 20, process_group=None):
         self.model = model
@@ -168,6 +175,7 @@ class DataParallelSGD:
                 loss = self.step(loss_fn)
 
             def replay():
+                _check_kernels()
                 graph.replay()
                 return loss
             replay.graph = graph
@@ -187,6 +195,7 @@ class DataParallelSGD:
             self._defer_allreduce = False
 
         def replay():
+            _check_kernels()
             fwd_bwd.replay()
             handles = [dist.all_reduce(b["flat"], op=dist.ReduceOp.SUM, group=self.group, async_op=True) for b in self.buckets]
             for h in handles:

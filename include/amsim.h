@@ -305,9 +305,13 @@ void amsim_debug_reload_env(void);
 int amsim_debug_bounds_report(unsigned long long* word);
 
 /* The tensor-core kernels bound every wait between their warps; one that runs out makes the kernel
- * end with wrong results instead of hanging.  This call waits for the device, returns nonzero in
- * *stuck if that has happened on the current device since the last call (it never should), and clears
- * the mark.  No reference counterpart. */
+ * end with wrong results instead of hanging (it never should).  The kernel leaves a mark in host
+ * memory, and the next call that takes a LUT on that device returns AMSIM_ERR_CUDA once, launching
+ * nothing.  amsim_async_status does nothing else: AMSIM_OK, or that error, without waiting for the
+ * device (for hosts that replay captured launches and make no other calls).
+ * amsim_debug_wait_report waits for the device, returns nonzero in *stuck if it has happened on
+ * the current device since it was last reported, and clears the mark.  No reference counterpart. */
+int amsim_async_status(void);
 int amsim_debug_wait_report(unsigned* stuck);
 
 /* Host-side check of the kernels' constant-divisor arithmetic (no GPU work):

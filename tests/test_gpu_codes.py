@@ -237,3 +237,21 @@ def test_every_shipped_table_takes_the_path(forced):
         assert not torch.equal(a, b), lut
         assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5
     assert np.isfinite(a.cpu().numpy()).all()
+
+
+def test_a_wait_that_runs_out_is_reported_by_the_next_call(forced, monkeypatch):
+    """With no tries at all every warp gives up at its first wait: the launch ends, and the next call says so, once."""
+    from approxtrain_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, w, lut = torch.randn(600, 300, generator=g, device="cuda"), torch.randn(300, 200, generator=g, device="cuda"), lut_path("MBM_7")
+    want = ops.denseam(x, w, lut)
+    monkeypatch.setenv("AMSIM_CODES_SPIN", "0")
+    forced.lib.amsim_debug_reload_env()
+    ops.denseam(x, w, lut)
+    torch.cuda.synchronize()
+    monkeypatch.delenv("AMSIM_CODES_SPIN")
+    forced.lib.amsim_debug_reload_env()
+    with pytest.raises(ops.AmsimError, match="gave up waiting"):
+        ops.denseam(x, w, lut)
+    assert torch.equal(ops.denseam(x, w, lut), want)      # (the tile counters are in step)
+    assert forced.lib.amsim_async_status() == 0
