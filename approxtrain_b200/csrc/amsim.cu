@@ -464,48 +464,139 @@ int scratch_alloc(cudaStream_t st, int device, size_t bytes, float** out) {
   return AMSIM_OK;
 }
 
-// Scratch of a balanced launch.  Outside a graph capture it is a stream-ordered allocation (safe for
-// launches on several streams at once).  While the stream is being captured nothing may be
-// allocated, so a capture uses one persistent buffer per device: every eager balanced launch makes
-// sure that buffer is at least as large as its own scratch (growing it is the one place where this
-// library calls cudaMalloc after a LUT is open; it happens a handful of times, on the first eager
-// steps), so a capture that follows a few warm-up steps of the same shapes finds room; a capture that
-// does not takes the plain / cluster launch instead.  The nodes of one captured stream run in order,
-// so they can share the buffer; graphs that are replayed concurrently on several streams must not
-// both contain balanced launches.
+// Scratch of a launch whose tiles are shared between CTAs.  Outside a graph capture it is a stream-ordered allocation (safe
+// for launches on several streams at once).  Captured launches use a region of their capture and their stream: launches
+// of one stream in one capture run in order and share it; forked branches, and graphs that are replayed at the same time,
+// have regions of their own.  A region is allocated while the stream is being captured (the calling thread's capture mode
+// is relaxed for that call) and belongs to the graph: when the graph and what was instantiated from it are gone it serves
+// the next capture, or is freed.
 struct BalancedScratch {
   float* ws = nullptr;
   bool pooled = false;
 };
-// The persistent buffer starts with room for the per-tile counters of a launch.  They are zeroed when
-// the buffer is created and the CTA that completes a tile puts its counter back to zero, so launches
-// inside a captured graph need no memset node.
-constexpr size_t kPersistentCounters = 1u << 16;
-constexpr size_t kPersistentCounterBytes = kPersistentCounters * sizeof(int);
+// A region starts with room for the per-tile counters of a launch.  A captured memset zeroes them when the stream's first
+// launch takes the region, and the CTA that completes a tile puts its counter back to zero: one memset node per stream.
+constexpr size_t kRegionCounters = 1u << 16;
+constexpr size_t kRegionCounterBytes = kRegionCounters * sizeof(int);
+constexpr size_t kMostSpareRegions = 4;  // kept per device for later captures
 
-int balanced_scratch_acquire(cudaStream_t st, int device, size_t bytes, bool capturing, BalancedScratch* out) {
-  static std::mutex mu;
-  static std::map<int, std::pair<void*, size_t>> persistent;
-  out->ws = nullptr;
-  out->pooled = false;
+struct CaptureRegion {
+  void* mem;
+  size_t bytes;
+  int device;
+  unsigned long long capture;
+  cudaStream_t stream;
+};
+struct CaptureRegions {
+  std::mutex mu;
+  std::vector<CaptureRegion*> used;   // by a capture or a graph; the newest of a stream last
+  std::vector<CaptureRegion*> spare;
+};
+CaptureRegions& capture_regions() {
+  static CaptureRegions* const r = new CaptureRegions;  // (graphs may outlive this library's statics)
+  return *r;
+}
+// Called when the last graph that held the region is gone, on a thread that must not call CUDA.
+void CUDART_CB region_released(void* p) {
+  CaptureRegions& r = capture_regions();
+  std::lock_guard<std::mutex> lk(r.mu);
+  r.used.erase(std::find(r.used.begin(), r.used.end(), static_cast<CaptureRegion*>(p)));
+  r.spare.push_back(static_cast<CaptureRegion*>(p));
+}
+
+// Calls that no capture allows in its strict modes: this thread's, for as long as the object lives, are allowed.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Frees the spare regions of the device beyond the bound.  (No CUDA call under the lock that region_released takes.)
+void free_spare_regions(int device) {
+  CaptureRegions& r = capture_regions();
+  std::vector<CaptureRegion*> gone;
   {
-    std::lock_guard<std::mutex> lk(mu);
-    auto& slot = persistent[device];
-    if (capturing) {
-      if (slot.first && slot.second >= bytes) out->ws = static_cast<float*>(slot.first);
-      return AMSIM_OK;  // ws stays null when there is no room: the caller launches without scratch
-    }
-    if (slot.second < bytes) {
-      void* fresh = nullptr;
-      if (cudaMalloc(&fresh, bytes) == cudaSuccess && cudaMemset(fresh, 0, kPersistentCounterBytes) == cudaSuccess) {
-        // the old buffer may still be referenced by instantiated graphs: it is kept, not freed
-        slot.first = fresh;
-        slot.second = bytes;
-      } else {
-        (void)cudaGetLastError();
-      }
+    std::lock_guard<std::mutex> lk(r.mu);
+    if (r.spare.size() <= kMostSpareRegions) return;
+    size_t kept = 0;
+    for (size_t i = r.spare.size(); i-- > 0;) {
+      if (r.spare[i]->device != device || ++kept <= kMostSpareRegions) continue;
+      gone.push_back(r.spare[i]);
+      r.spare.erase(r.spare.begin() + i);
     }
   }
+  RelaxedCapture relaxed;
+  for (CaptureRegion* g : gone) {
+    cudaFree(g->mem);
+    delete g;
+  }
+}
+
+// A region for the launches of a stream that is being captured; null when none can be had.
+void* capture_region(cudaStream_t st, int device, size_t bytes) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(st, &status, &id, &graph) != cudaSuccess || status != cudaStreamCaptureStatusActive || !graph) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  CaptureRegions& r = capture_regions();
+  CaptureRegion* region = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(r.mu);
+    for (size_t i = r.used.size(); i-- > 0;)
+      if (r.used[i]->capture == id && r.used[i]->stream == st && r.used[i]->device == device && r.used[i]->bytes >= bytes)
+        return r.used[i]->mem;
+    for (size_t i = 0; i < r.spare.size() && !region; ++i)
+      if (r.spare[i]->device == device && r.spare[i]->bytes >= bytes) {
+        region = r.spare[i];
+        r.spare.erase(r.spare.begin() + i);
+      }
+  }
+  if (!region) {
+    // as large as any tensor-core launch takes, so that a stream rarely needs a second one
+    const size_t size = std::max(bytes, kRegionCounterBytes + (size_t)sm_count(device) * code_tile(0).slot_bytes + (1u << 20));
+    RelaxedCapture relaxed;
+    void* mem = nullptr;
+    if (cudaMalloc(&mem, size) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    region = new CaptureRegion{mem, size, device, 0, nullptr};
+  }
+  region->capture = id;
+  region->stream = st;
+  {
+    std::lock_guard<std::mutex> lk(r.mu);
+    r.used.push_back(region);
+  }
+  cudaUserObject_t owner = nullptr;
+  if (cudaUserObjectCreate(&owner, region, region_released, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    (void)cudaGetLastError();
+    region_released(region);
+    return nullptr;
+  }
+  if (cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    (void)cudaGetLastError();
+    cudaUserObjectRelease(owner, 1);  // (hands the region back)
+    return nullptr;
+  }
+  if (cudaMemsetAsync(region->mem, 0, kRegionCounterBytes, st) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  return region->mem;
+}
+
+int balanced_scratch_acquire(cudaStream_t st, int device, size_t bytes, bool capturing, BalancedScratch* out) {
+  out->ws = nullptr;
+  out->pooled = false;
+  if (capturing) {
+    out->ws = static_cast<float*>(capture_region(st, device, bytes));
+    return AMSIM_OK;  // (null: the caller launches without scratch)
+  }
+  free_spare_regions(device);
   if (scratch_alloc(st, device, bytes, &out->ws) != AMSIM_OK) {
     (void)cudaGetLastError();
     out->ws = nullptr;
@@ -565,7 +656,7 @@ int launch_gather_t(cudaStream_t st, Params& p, int batch, int device) {
   // Fast mode, balanced launch: the plain grid would leave the last wave of resident CTA slots
   // partly empty (or never fill them), so the (tile, reduction block) pairs are dealt out in
   // equal runs to exactly as many CTAs as the device holds.  While the stream is being
-  // captured into a graph the scratch is a persistent buffer (see balanced_scratch_acquire).
+  // captured into a graph the scratch belongs to the graph (see balanced_scratch_acquire).
   // (not for tables in global memory: those launches are bound by L2 gathers, and lock-step CTAs
   // measured 50 % slower there)
   if constexpr (!EXACT && !lm_global(LM)) {
@@ -597,7 +688,7 @@ int launch_gather_t(cudaStream_t st, Params& p, int batch, int device) {
     // blocks) take the cluster split below instead, which adds partial tiles through distributed
     // shared memory rather than through parked tiles in global memory: the replayed LeNet-5 step
     // measured 4 % faster that way; anything larger is faster balanced (ResNet-50 +2 %,
-    // LeNet-300-100 +3 %; the persistent scratch needs no memset node).
+    // LeNet-300-100 +3 %; their scratch needs no memset node of its own).
     const bool capturing = cap != cudaStreamCaptureStatusNone;
     bool tiny = ctas * 2 <= slots && nkb >= 4 && iters <= 64;
     if (sw().capture_cluster >= 0) tiny = sw().capture_cluster != 0 && ctas * 2 <= slots && nkb >= 4;
@@ -609,15 +700,15 @@ int launch_gather_t(cudaStream_t st, Params& p, int batch, int device) {
       p.sk_grid = (int)grid;
       const size_t slot_bytes = (size_t)grid * 2 * TR * TC * L::NT * sizeof(float);
       // [counters kept at zero between launches][parked tiles][counters of a launch with more tiles than that]
-      const size_t bytes = kPersistentCounterBytes + slot_bytes + (size_t)ctas * sizeof(int);
+      const size_t bytes = kRegionCounterBytes + slot_bytes + (size_t)ctas * sizeof(int);
       BalancedScratch sc;
       rc = balanced_scratch_acquire(st, device, bytes, capturing, &sc);
       if (rc) return rc;
       if (sc.ws) {
         char* base = reinterpret_cast<char*>(sc.ws);
-        p.ws = reinterpret_cast<float*>(base + kPersistentCounterBytes);
-        const bool clean = !sc.pooled && (size_t)ctas <= kPersistentCounters;  // persistent buffer: zero already
-        p.sk_count = reinterpret_cast<int*>(clean ? base : base + kPersistentCounterBytes + slot_bytes);
+        p.ws = reinterpret_cast<float*>(base + kRegionCounterBytes);
+        const bool clean = !sc.pooled && (size_t)ctas <= kRegionCounters;  // a capture's region: zero already
+        p.sk_count = reinterpret_cast<int*>(clean ? base : base + kRegionCounterBytes + slot_bytes);
         fill_bounds(p, device, base, bytes);
         cudaError_t e1 = clean ? cudaSuccess : cudaMemsetAsync(p.sk_count, 0, (size_t)ctas * sizeof(int), st);
         if (e1 == cudaSuccess) {
@@ -632,7 +723,7 @@ int launch_gather_t(cudaStream_t st, Params& p, int batch, int device) {
         CUDA_TRY(e2);
         return AMSIM_OK;
       }
-      // no scratch to be had (pool exhausted, or a capture without a warm-up): the plain grid needs none
+      // no scratch to be had (out of memory): the plain grid needs none
       p.ws = nullptr;
     }
   }
@@ -817,18 +908,18 @@ int launch_gather(cudaStream_t st, Params& p, int batch, bool exact, int device)
     if (f.use) {
       cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
       CUDA_TRY(cudaStreamIsCapturing(st, &cap));
-      const size_t bytes = kPersistentCounterBytes + f.slot_bytes + f.counter_bytes;
+      const size_t bytes = kRegionCounterBytes + f.slot_bytes + f.counter_bytes;
       BalancedScratch sc;
       int rc = balanced_scratch_acquire(st, device, bytes, cap != cudaStreamCaptureStatusNone, &sc);
       if (rc) return rc;
       if (sc.ws) {
         char* base = reinterpret_cast<char*>(sc.ws);
-        const bool clean = !sc.pooled && (size_t)f.tiles * 2 <= kPersistentCounters;
-        char* counters = clean ? base : base + kPersistentCounterBytes + f.slot_bytes;
+        const bool clean = !sc.pooled && (size_t)f.tiles * 2 <= kRegionCounters;
+        char* counters = clean ? base : base + kRegionCounterBytes + f.slot_bytes;
         Params q = p;
         fill_bounds(q, device, base, bytes);
         cudaError_t e1 = clean ? cudaSuccess : cudaMemsetAsync(counters, 0, f.counter_bytes, st);
-        rc = e1 == cudaSuccess ? launch_codes(st, q, f, false, counters, base + kPersistentCounterBytes, device) : AMSIM_OK;
+        rc = e1 == cudaSuccess ? launch_codes(st, q, f, false, counters, base + kRegionCounterBytes, device) : AMSIM_OK;
         const cudaError_t e2 = balanced_scratch_release(st, sc);
         CUDA_TRY(e1);
         if (rc) return rc;

@@ -255,3 +255,65 @@ def test_a_wait_that_runs_out_is_reported_by_the_next_call(forced, monkeypatch):
         ops.denseam(x, w, lut)
     assert torch.equal(ops.denseam(x, w, lut), want)      # (the tile counters are in step)
     assert forced.lib.amsim_async_status() == 0
+
+
+def _products(n, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [(torch.randn(1200 + 100 * i, 700, generator=g, device="cuda"), torch.randn(700, 300, generator=g, device="cuda"))
+            for i in range(n)]
+
+
+@pytest.mark.parametrize("codes", [1, 0])
+def test_captured_launches_on_forked_branches_do_not_share_scratch(forced, codes):
+    """Tiles of one branch parked among the other's would show as wrong sums; eager launches have scratch of their own."""
+    from approxtrain_b200 import ops
+    lut = lut_path("MBM_7")
+    _on(forced, codes, lambda: None)
+    pairs = _products(4, 1)
+    want = [ops.denseam(x, w, lut) for x, w in pairs]
+    torch.cuda.synchronize()
+    graph, out = torch.cuda.CUDAGraph(), [None] * len(pairs)
+    side = [torch.cuda.Stream() for _ in pairs[1:]]
+    with torch.cuda.graph(graph):
+        here = torch.cuda.current_stream()
+        for i, s in enumerate(side):
+            s.wait_stream(here)
+            with torch.cuda.stream(s):
+                out[i + 1] = ops.denseam(*pairs[i + 1], lut)
+                out[i + 1] = ops.denseam(*pairs[i + 1], lut)     # (a second launch of the stream takes the same region)
+        out[0] = ops.denseam(*pairs[0], lut)
+        for s in side:
+            here.wait_stream(s)
+    for _ in range(20):
+        for o in out:
+            o.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(out, want))
+
+
+def test_graphs_replayed_side_by_side_do_not_share_scratch_and_give_it_back(forced):
+    from approxtrain_b200 import ops
+    lut = lut_path("MIT_7")
+    pairs = _products(2, 2)
+    want = [ops.denseam(x, w, lut) for x, w in pairs]
+    free = []
+    for round_ in range(8):
+        graphs, outs = [], []
+        for x, w in pairs:
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[-1]):
+                outs.append(ops.denseam(x, w, lut))
+        streams = [torch.cuda.Stream() for _ in pairs]
+        for _ in range(10):
+            for s, gr in zip(streams, graphs):
+                s.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(s):
+                    gr.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(outs, want))
+        del graphs, outs, gr
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert min(free[2:]) >= free[1] - (4 << 20), free      # later captures use what earlier graphs gave back
