@@ -107,3 +107,65 @@ def test_bounds_checking_build_sees_no_out_of_range_access():
     assert out.returncode == 0, (out.stdout + out.stderr)[-4000:]
     assert "all accesses in bounds" in out.stdout
     print(out.stdout.strip().splitlines()[-1])
+
+
+CODES_CHILD = CHILD[:CHILD.index("n_cases = 0")] + r'''
+os.environ["AMSIM_CODES"] = "1"
+_lib.lib.amsim_debug_reload_env()
+def off(t):                     # a copy that starts four bytes after a 16-byte boundary
+    v = torch.empty(t.numel() + 1, device="cuda")[1:].view(t.shape); v.copy_(t); return v
+n_cases = 0
+for shape in SHAPES + [(2, 14, 14, 37, 5, 5, 257), (1, 30, 30, 3, 7, 7, 64), (4, 20, 20, 64, 3, 3, 129)]:
+    n, h, w, c, kh, kw, k = shape
+    for stride, pad in ((1, "SAME"), (2, "SAME"), (1, "VALID"), (2, "VALID")):
+        if pad == "VALID" and (kh > h or kw > w): continue
+        for lname in ("MBM_7", "MIT_7", "MIT_5"):
+            lut, m = load_lut(lut_path(lname))
+            rng = np.random.default_rng(zlib.crc32(repr((shape, stride, pad, lname)).encode()))
+            x = rng.standard_normal((n, h, w, c)).astype(np.float32); x[x < -0.5] = 0
+            wt = rng.standard_normal((kh, kw, c, k)).astype(np.float32)
+            g = o.geometry(n, h, w, c, kh, kw, k, stride, stride, pad)
+            dy = rng.standard_normal((n, g.out_h, g.out_w, k)).astype(np.float32)
+            kw_ = dict(strides=[1, stride, stride, 1], padding=pad, mant_mul_lut=lut_path(lname))
+            refs = (o.conv2d_fwd(g, x, wt, lut, m), o.conv2d_bwd_filter(g, x, dy, lut, m), o.conv2d_bwd_input(g, wt, dy, lut, m))
+            for f in (lambda t: t, off):
+                X, W, D = f(dev(x)), f(dev(wt)), f(dev(dy))
+                outs = (ops.convam(X, W, **kw_), ops.convam_filter_grad(wt.shape, X, D, **kw_), ops.convam_input_grad(x.shape, W, D, **kw_))
+                v = verdict()
+                assert v == 0, f"out-of-bounds access: line {v >> 44} buffer {((v >> 40) & 15) - 1} offset {v & ((1 << 40) - 1)} in {shape} s{stride} {pad} {lname}"
+                for got, want in zip(outs, refs):
+                    assert rel_l2(got.cpu().numpy(), want) <= 1e-5
+                n_cases += 1
+            X[0, 2, 2, 0] = 2.0 ** 100; W[0, 0, 0, 1] = 2.0 ** 26; D[0, -1, -1, 1] = 2.0 ** 26     # outputs that are recomputed
+            ops.convam(X, W, **kw_); ops.convam_filter_grad(wt.shape, X, D, **kw_); ops.convam_input_grad(x.shape, W, D, **kw_)
+            assert verdict() == 0
+lp = lut_path("MBM_7")
+rng = np.random.default_rng(1)
+for b, kin, u in ((7, 33, 5), (130, 64, 129), (256, 100, 10), (1, 1, 1), (300, 64, 72), (1500, 700, 300)):
+    x = rng.random((b, kin)).astype(np.float32); wm = rng.standard_normal((kin, u)).astype(np.float32)
+    gy = rng.standard_normal((b, u)).astype(np.float32)
+    ops.denseam(dev(x), dev(wm), lp); ops.denseam_grad(dev(gy), dev(x), dev(wm), lp)
+    assert verdict() == 0
+for sa, sb, ta, tb in (((4, 16, 24), (4, 24, 8), False, False), ((16, 24), (3, 24, 8), False, False), ((3, 24, 16), (3, 8, 24), True, True),
+                       ((6, 130, 64), (6, 70, 64), False, True)):
+    a = dev(rng.standard_normal(sa).astype(np.float32)); bb = dev(rng.standard_normal(sb).astype(np.float32))
+    ops.matmulam(a, bb, transpose_a=ta, transpose_b=tb, mant_mul_lut=lp)
+    assert verdict() == 0
+os.environ["AMSIM_BOUNDS_SHRINK"] = "64"
+_lib.lib.amsim_debug_reload_env()
+ops.denseam(dev(rng.random((300, 64)).astype(np.float32)), dev(rng.random((64, 72)).astype(np.float32)), lp)
+v = verdict()
+assert v != 0 and ((v >> 40) & 15) - 1 == 2, hex(v)      # the last stores of the output
+print(f"tensor-core path, bounds-checked cases: {n_cases}, all accesses in bounds")
+'''
+
+
+def test_bounds_checking_build_on_the_tensor_core_path():
+    """Every case forced onto code_gemm, aligned and not; scratch, counters and recomputed outputs included."""
+    from approxtrain_b200 import _build
+    if not os.path.exists(_build.CHECKED_LIB_PATH):
+        pytest.skip("libamsim_check.so not built (approxtrain_b200._build.build_checked)")
+    env = dict(os.environ, AMSIM_LIBRARY=_build.CHECKED_LIB_PATH, AMSIM_REPO=ROOT)
+    out = subprocess.run([sys.executable, "-c", CODES_CHILD], capture_output=True, text=True, timeout=1500, env=env, cwd=ROOT)
+    assert out.returncode == 0, (out.stdout + out.stderr)[-4000:]
+    assert "all accesses in bounds" in out.stdout

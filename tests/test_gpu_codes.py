@@ -317,3 +317,79 @@ def test_graphs_replayed_side_by_side_do_not_share_scratch_and_give_it_back(forc
         torch.cuda.empty_cache()
         free.append(torch.cuda.mem_get_info()[0])
     assert min(free[2:]) >= free[1] - (4 << 20), free      # later captures use what earlier graphs gave back
+
+
+SOME = [(2, 9, 13, 16, 3, 3, 65, 1, "SAME"), (1, 30, 30, 3, 7, 7, 64, 2, "VALID"), (3, 11, 7, 8, 3, 3, 129, 2, "SAME"), (2, 14, 14, 64, 1, 1, 300, 1, "VALID")]
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7"])
+@pytest.mark.parametrize("shape", SOME)
+def test_fused_epilogue_equals_the_separate_operations(forced, lut, shape):
+    from approxtrain_b200 import ops
+    n, h, w, c, kh, kw, k, s, pad = shape
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x, wt = torch.randn(n, h, w, c, generator=g, device="cuda"), torch.randn(kh, kw, c, k, generator=g, device="cuda")
+    b, sc = torch.randn(k, generator=g, device="cuda"), torch.rand(k, generator=g, device="cuda") - 0.3
+    kw_ = dict(strides=s, padding=pad, mant_mul_lut=lut_path(lut))
+    y = ops.convam(x, wt, **kw_)
+    assert torch.equal(ops.convam_bias_act(x, wt, b, activation="relu", scale=sc, **kw_), torch.relu(y * sc + b))
+    assert torch.equal(ops.convam_bias_act(x, wt, b, **kw_), y + b)
+    if kh == 1:
+        flat, mat = x.reshape(-1, c), wt[0, 0]
+        assert torch.equal(ops.denseam_bias_act(flat, mat, b, activation="relu", mant_mul_lut=lut_path(lut)),
+                           torch.relu(ops.denseam(flat, mat, lut_path(lut)) + b))
+
+
+def _off_by_one_float(t):
+    room = torch.empty(t.numel() + 1, device="cuda")
+    view = room[1:].view(t.shape)
+    view.copy_(t)
+    assert view.data_ptr() % 16 == 4
+    return view
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_5"])
+@pytest.mark.parametrize("shape", SOME)
+def test_operands_off_16_byte_alignment(forced, lut, shape):
+    """Element-wise fetches of what aligned operands fetch 16 bytes at a time: the same sums in the same order."""
+    from approxtrain_b200 import ops
+    n, h, w, c, kh, kw, k, s, pad = shape
+    g = torch.Generator(device="cuda").manual_seed(c)
+    x, wt = torch.randn(n, h, w, c, generator=g, device="cuda"), torch.randn(kh, kw, c, k, generator=g, device="cuda")
+    kw_ = dict(strides=s, padding=pad, mant_mul_lut=lut_path(lut))
+    y = ops.convam(x, wt, **kw_)
+    dy = torch.randn(y.shape, generator=g, device="cuda")
+    dx, dw = ops.convam_input_grad(x.shape, wt, dy, **kw_), ops.convam_filter_grad(wt.shape, x, dy, **kw_)
+    for f in (lambda t: t, _off_by_one_float):
+        for e in (lambda t: t, _off_by_one_float):
+            assert torch.equal(ops.convam(f(x), e(wt), **kw_), y)
+            assert torch.equal(ops.convam_input_grad(x.shape, e(wt), f(dy), **kw_), dx)
+            assert torch.equal(ops.convam_filter_grad(wt.shape, f(x), e(dy), **kw_), dw)
+
+
+@pytest.mark.parametrize("lut", ["MBM_7", "MIT_7", "MBM_5"])
+@pytest.mark.parametrize("rows,width,units", [(300, 64, 257), (257, 500, 64), (130, 33, 300), (1000, 129, 130)])
+def test_dense_gradients_in_either_operand_role(forced, lut, rows, width, units):
+    from approxtrain_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, w = torch.randn(rows, width, generator=g, device="cuda"), torch.randn(width, units, generator=g, device="cuda")
+    dy = torch.randn(rows, units, generator=g, device="cuda")
+    for got, want in zip(ops.denseam_grad(dy, x, w, lut_path(lut)), ops.denseam_grad(dy, x, w, lut_path(lut), deterministic=True)):
+        _close(got, want)
+
+
+def test_offsets_beyond_31_bits(forced):
+    from approxtrain_b200 import ops
+    rows = (1 << 31) // 64 + 5000
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs 40 GB")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w = torch.randn(64, 64, generator=g, device="cuda")
+    x = torch.randn(rows, 64, generator=g, device="cuda")
+    y = ops.denseam(x, w, lut_path("MBM_7"))
+    for part in (slice(0, 3000), slice(rows // 2, rows // 2 + 3000), slice(rows - 3000, rows)):
+        _close(y[part], ops.denseam(x[part], w, lut_path("MBM_7"), deterministic=True))
+    dw = ops.denseam_grad(y, x, w, lut_path("MBM_7"))[1]        # the reduction runs over all rows
+    want = sum(ops.denseam_grad(y[i:i + rows // 4 + 1], x[i:i + rows // 4 + 1], w, lut_path("MBM_7"))[1].double()
+               for i in range(0, rows, rows // 4 + 1))
+    _close(dw, want)
