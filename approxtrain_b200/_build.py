@@ -24,7 +24,7 @@ NVCC_FLAGS = [
 ]
 
 
-def _compile(out: str, extra=(), only_stale=False) -> None:
+def _compile(out: str, extra=()) -> None:
     """The sources side by side (one nvcc each), then one link."""
     nvcc = os.environ.get("NVCC", "nvcc")
     tmp = os.path.join(_PKG, "build", os.path.basename(out))
@@ -33,9 +33,6 @@ def _compile(out: str, extra=(), only_stale=False) -> None:
     for src in SOURCES:
         obj = os.path.join(tmp, os.path.basename(src) + ".o")
         objs.append(obj)
-        deps = [src] + HEADERS
-        if only_stale and os.path.exists(obj) and all(os.path.getmtime(d) <= os.path.getmtime(obj) for d in deps):
-            continue
         jobs.append((src, subprocess.Popen([nvcc] + NVCC_FLAGS + list(extra) + ["-c", "-o", obj, src])))
     failed = [src for src, job in jobs if job.wait() != 0]
     if failed:

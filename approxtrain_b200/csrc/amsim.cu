@@ -838,9 +838,10 @@ CodePlan plan_codes(int P, int Q, int K, int batch, int sms, const CodeTraits& t
   f.grid = (int)std::min<double>((double)std::min<long long>(sms / 2, std::max<long long>(1, f.iters / 2)), std::max(1.0, best));
   if (f.grid < 1) return f;
   // Below 1e8 products both paths take a few tens of microseconds, and the estimates do not tell them apart.
-  // Batched products stay on the table kernels: attention cuts softmax weights down to the table's few mantissa bits for
-  // its next product, so a last-bit change of the scores shows as 2e-3 of the result's root mean square there; and a
-  // tile's 256 rows are of one product (512 of 128 x 128 x 64: MIT_7 65 / 137 us, MBM_7 109 / 88 us).
+  // Batched products stay on the table kernels.  Attention cuts softmax weights down to the table's few mantissa bits for
+  // its next product, so a last-bit change of the scores shows as 2e-3 of the result's root mean square there, and a call
+  // does not say what its result feeds.  A tile's 256 rows are of one product, too: 512 of 128 x 128 x 64 take MIT_7 65 / 137 us,
+  // MBM_7 109 / 88 us.  (Few and large ones would gain: 2 x 4096 x 1024 x 1024, MBM_7, estimated 1451 / 312 us.)
   const double products = (double)P * Q * K * batch;
   if (w.codes < 0 && (batch > 1 || products < 1e8 || K < code_least_k(t.slots) || code_us(f, t) > 0.95 * table_us(products, K, t))) return f;
   f.slot_bytes = (size_t)f.grid * 2 * tile.slot_bytes;
