@@ -24,13 +24,19 @@
  *                        except where an operand has a zero exponent field
  *                        (product taken as 0) or the exponent sum is <= 127
  *                        (reference returns 0, here the exact tiny product,
- *                        < 2^-125); each forward / input-gradient output is one
- *                        ascending-k FP32 chain like the reference kernel, the
- *                        filter / weight gradients are split along the
- *                        reduction and summed in a fixed order, and so are
- *                        forward / input-gradient outputs of shapes with too
- *                        few output tiles to fill the GPU (thread-block clusters
- *                        share a tile's reduction).  Run-to-run identical.
+ *                        < 2^-125) or exceeds 2^128.  Sums are FP32 in a fixed
+ *                        order, run to run identical: one ascending-k chain as in
+ *                        the reference kernel for forward / input-gradient outputs
+ *                        of plain launches; partial chains added in a fixed order
+ *                        for filter / weight gradients and for tiles that thread
+ *                        blocks share.  Unbatched products of 1e8 multiplications
+ *                        and more over a table that factors over 4-bit floats
+ *                        (every shipped one) may run on the tensor cores, whose
+ *                        accumulators truncate: with operands of ordinary spread no
+ *                        further from the exact sums than the chains, with
+ *                        magnitudes spread over 2^20 up to 4e-6 (chains 5e-7).
+ *                        There an operand with exponent field 255 makes every
+ *                        output that it takes part in NaN.
  *   AMSIM_DETERMINISTIC  every product is the reference primitive bit for bit
  *                        (cuda/AMsimulator.inl:13-36) and every output is one
  *                        ascending chain in the reference's order
