@@ -77,7 +77,7 @@ struct Switches {
   int capture_cluster = -1; // AMSIM_CAPTURE_CLUSTER=0/1 small launches inside a graph capture: balanced / cluster split
   int balanced_waves = -1;  // AMSIM_BALANCED_WAVES=n    CTAs of a balanced launch: n times the resident slots
   int codes = -1;           // AMSIM_CODES=0/1           tensor-core path of factorable tables: never / whenever eligible
-  int codes_spin = -1;      // AMSIM_CODES_SPIN=n        tries of a wait in that path's kernels (0: the first wait gives up)
+  int codes_spin = -1;      // AMSIM_CODES_SPIN=0        no tries of a wait in that path's kernels: the first one gives up
   int bounds_shrink = 0;    // AMSIM_BOUNDS_SHRINK=n     bounds-checking build only: the output's recorded extent is n bytes
                             //                           short, so its last stores are caught (self-test of the checker)
 };
@@ -865,7 +865,7 @@ void code_params(CodeParams& c, const Params& p, const CodePlan& f, bool fgrad) 
   c.sh_u = p.ct_sh_u;
   c.unit = p.ct_unit;
   c.fgrad = fgrad ? 1 : 0;
-  c.spins = sw().codes_spin >= 0 ? sw().codes_spin : CT_MAXSPIN;
+  c.no_tries = sw().codes_spin == 0;
   c.chunk = f.chunk;
   const bool va = aligned16(p.V) && p.v_bs % 4 == 0;
   if (fgrad) c.v_mode = va && p.g.SC % 4 == 0 ? CT_RVEC : CT_RSCL;
